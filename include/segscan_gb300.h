@@ -171,10 +171,14 @@ ss_status ss_spmm_rbpr(const ss_csr *A, int N, const void *B, void *C,
 
 /* Replaces csrspmm_rowcaching_nnzbalance_cg<Index, DType, group_factor,
  * thread_per_block, CoarsenFactor, ThreadNz, block_numer, block_denom>
- * (spmm_cg.cuh:553-555).  Chunks (ThreadNz * 2^group_factor nonzeros)
- * smaller than the nonzeros' share per resident group of one full wave are
- * merged up to that share (also for ebpr); the result is the same up to
- * FP32 rounding order, deterministic for given inputs and knobs. */
+ * (spmm_cg.cuh:553-555).  Tuples that ask for chunks (ThreadNz *
+ * 2^group_factor nonzeros) of up to 2048 nonzeros run the tile walk, whose
+ * lanes, vectors and pieces follow from N, the types and the alignment;
+ * longer chunks (and a workspace that only the group walk fits) run the
+ * group walk with those chunks, merged up to the nonzeros' share per
+ * resident group of one full wave where they are smaller (as for ebpr).
+ * The result is the same up to FP32 rounding order, deterministic for given
+ * inputs, alignment and knobs. */
 ss_status ss_spmm_ebsr(const ss_csr *A, int N, const void *B, void *C,
                        int c_dtype, int accumulate, const ss_knobs *knobs,
                        void *ws, size_t ws_bytes, void *stream);
@@ -346,9 +350,10 @@ void ss_mtx_free(ss_mtx *m);
  * coarsen_factor and thread_per_block come from per_mat[0] (NULL = ebsr
  * defaults).  ss_batch_plan uploads the plan and synchronises the stream.
  * ss_spmm_batched then computes C[m] = A[m] * B[m] for every m in one
- * persistent launch (after one memset of its counters; rows that straddle
- * work items are assembled inside that launch), stream-ordered (it can be
- * replayed from a captured CUDA graph).  Not in the reference. */
+ * launch (after one memset of its counters; rows that straddle work items
+ * are assembled inside that launch), or two when the batch has both
+ * element-balanced matrices and row-balanced or long-chunk ones,
+ * stream-ordered (it can be replayed from a captured CUDA graph).  Not in the reference. */
 ss_status ss_batch_plan_size(int count, const ss_csr *mats, int N,
                              const ss_knobs *per_mat, size_t *host_bytes,
                              size_t *dev_bytes);

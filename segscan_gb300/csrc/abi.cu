@@ -309,6 +309,10 @@ static ss_status make_spmm_call(int strategy, const ss_csr *A, int N, const void
 // cheaper there; the sums are the same (0 + x = x).
 static bool hypersparse(long long nnz, long long rows) { return 2 * nnz < rows; }
 
+static bool takes_tile(const ss_knobs &k, int N, int nnz, int dtype) {
+  return tile_tuple(k.group_factor, k.thread_nz) && tile_fits(N, nnz, dtype);
+}
+
 // Vector accesses need the B/C row starts aligned to V elements.
 static ss_status check_vec_alignment(const void *B, const void *C, int es, int cs, int V) {
   if (((uintptr_t)B % (size_t)(es * V)) || ((uintptr_t)C % (size_t)(cs * V)))
@@ -324,6 +328,14 @@ static ss_status spmm_geometry(int strategy, const SpmmCall &c, const ss_knobs &
     case SS_EBPR: return geom_pr(c.M, c.nnz, c.N, c.val_dtype, k, eg);
   }
   return fail(SS_ERR_INVALID_ARG, "unknown strategy %d", strategy);
+}
+
+size_t ebsr_walk_workspace(const ss_csr *A, int N, const ss_knobs *knobs) {
+  ss_knobs tmp;
+  const ss_knobs *k = knobs_or_default(SS_EBSR, N, knobs, tmp);
+  EbGeom g;
+  if (!k || geom_sr(A->nrow, A->nnz, N, A->value_dtype, dtype_size(A->value_dtype), *k, g) != SS_OK) return (size_t)-1;
+  return eb_workspace_bytes(g, N);
 }
 
 }  // namespace ss
@@ -402,6 +414,8 @@ ss_status ss_spmm_workspace_size(int strategy, const ss_csr *A, int N, const ss_
   st = spmm_geometry(strategy, c, *k, rg, eg);
   if (st) return st;
   *bytes = (strategy == SS_EBSR || strategy == SS_EBPR) ? eb_workspace_bytes(eg, N) : 0;
+  if (strategy == SS_EBSR && A->nnz > 0 && N > 0 && takes_tile(*k, N, A->nnz, A->value_dtype))
+    *bytes = tile_workspace_bytes(N, A->nnz, A->value_dtype);
   return SS_OK;
 }
 
@@ -430,7 +444,15 @@ ss_status ss_spmm(int strategy, const ss_csr *A, int N, const void *B, void *C, 
       cudaError_t e = cudaMemsetAsync(C, 0, (size_t)c.M * c.N * dtype_size(c.c_dtype), s);
       return e == cudaSuccess ? SS_OK : cuda_fail(e, "zero C");
     }
-    const size_t need = eb_workspace_bytes(eg, N);
+    size_t need = eb_workspace_bytes(eg, N);
+    bool tile = false;
+    if (strategy == SS_EBSR && takes_tile(*k, N, c.nnz, c.val_dtype)) {
+      // a workspace sized for the group walk (the fixed scratch of
+      // ss_spmm_ebsr_noalloc, a caller's own constant) still gets that walk
+      const size_t tneed = tile_workspace_bytes(N, c.nnz, c.val_dtype);
+      tile = ws_bytes >= tneed;
+      if (tile || tneed < need) need = tneed;
+    }
     if (ws_bytes < need || (need > 0 && (!ws || ((uintptr_t)ws % 256))))
       return fail(SS_ERR_WORKSPACE, "workspace needs %zu bytes (256-byte aligned), got %zu", need, ws_bytes);
     if (!accumulate && hypersparse(c.nnz, c.M)) {
@@ -440,6 +462,7 @@ ss_status ss_spmm(int strategy, const ss_csr *A, int N, const void *B, void *C, 
       if (e != cudaSuccess) return cuda_fail(e, "zero C");
       c.accumulate = 1;
     }
+    if (tile) return launch_ebsr_tile(c, ws, s);
     return strategy == SS_EBSR ? launch_ebsr(c, eg, ws, s) : launch_ebpr(c, eg, ws, s);
   }
   return strategy == SS_RBSR ? launch_rbsr(c, rg, s) : launch_rbpr(c, rg, s);

@@ -13,9 +13,10 @@ static size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 // Fills h (everything but the offsets' final sizes) and per-matrix chunk
 // sizes; returns the number of items.
 // strategies: per matrix SS_EBSR (element-balanced chunks) or SS_RBSR
-// (blocks of whole rows), null = all SS_EBSR.
+// (blocks of whole rows), null = all SS_EBSR.  vmax: elements per vector the
+// alignment of every B and C allows (the tile walk's vector).
 static ss_status batch_layout(int count, const ss_csr *mats, int N, const ss_knobs *per_mat, const int *strategies,
-                              BatchHeader &h, std::vector<BatchMat> *out) {
+                              int vmax, BatchHeader &h, std::vector<BatchMat> *out, std::vector<TileProb> *tout) {
   if (count < 1 || !mats || N < 1) return fail(SS_ERR_INVALID_ARG, "batch needs count >= 1, N >= 1 and matrices");
   const int dt = mats[0].value_dtype;
   ss_knobs k0;
@@ -40,7 +41,12 @@ static ss_status batch_layout(int count, const ss_csr *mats, int N, const ss_kno
   h.block = g.block;
   h.smem = g.smem;
   h.kahan = k0.kahan_threshold > 0 ? k0.kahan_threshold : 1024;
-  long long items = 0;
+  const TileGeom tg0 = tile_geom(N, 0, dt, vmax);
+  h.tG = tg0.G;
+  h.tV = tg0.V;
+  h.tNV = tg0.NV;
+  h.tphases = tg0.phases;
+  long long items = 0, titems = 0;
   for (int m = 0; m < count; m++) {
     const ss_csr &A = mats[m];
     if (A.nrow < 0 || A.ncol < 0 || A.nnz < 0 || (A.nrow > 0 && !A.indptr) || (A.nnz > 0 && !A.indices))
@@ -57,7 +63,7 @@ static ss_status batch_layout(int count, const ss_csr *mats, int N, const ss_kno
     bm.K = A.ncol;
     bm.nnz = A.nnz;
     bm.chunk = tnz * h.G;
-    bm.num_chunks = A.nnz > 0 ? ceil_div(A.nnz, bm.chunk) : (A.nrow > 0 ? 1 : 0);
+    bm.num_chunks = A.nnz > 0 ? ceil_div(A.nnz, bm.chunk) : 0;
     const int strategy = strategies ? strategies[m] : SS_EBSR;
     if (strategy != SS_EBSR && strategy != SS_RBSR)
       return fail(SS_ERR_UNSUPPORTED_KNOBS, "matrix %d: batched strategy %d is neither SS_EBSR nor SS_RBSR", m,
@@ -68,23 +74,45 @@ static ss_status batch_layout(int count, const ss_csr *mats, int N, const ss_kno
       bm.rows_per_item = (int)std::min<long long>(std::max(1LL, rows), (long long)A.nrow);
       bm.num_chunks = ceil_div(A.nrow, bm.rows_per_item);
     }
+    if (A.nrow > 0 && (A.nnz == 0 || (strategy == SS_EBSR && tile_tuple(h.log2G, tnz) && tile_fits(N, A.nnz, dt)))) {
+      const TileGeom g = tile_geom(N, A.nnz, dt, vmax);
+      TileProb p;
+      memset(&p, 0, sizeof(p));
+      p.indptr = A.indptr; p.cols = A.indices; p.vals = A.values;
+      p.M = A.nrow; p.K = A.ncol; p.nnz = A.nnz;
+      p.slog = g.slog;
+      p.item_begin = (int)titems;
+      p.wide = (((uintptr_t)A.indices | (uintptr_t)A.values) & 15u) == 0;
+      p.index = m;
+      titems += g.tiles;
+      h.tsmem = std::max(h.tsmem, g.smem);
+      h.tile_count++;
+      if (tout) tout->push_back(p);
+      bm.num_chunks = 0;
+    }
     bm.item_begin = (int)items;
     bm.use_tma = (((uintptr_t)A.indices & 15u) == 0) && (A.values == nullptr || ((uintptr_t)A.values & 15u) == 0) &&
                  (bm.chunk % 8) == 0;
     items += bm.num_chunks;
-    if (items > 0x7fffffffLL) return fail(SS_ERR_CAPACITY, "too many work items");
+    if (items > 0x7fffffffLL || titems * h.tphases > 0x7fffffffLL) return fail(SS_ERR_CAPACITY, "too many work items");
     if (out) out->push_back(bm);
   }
   h.total_items = (int)items;
+  h.tile_items = (int)titems;
   size_t o = 0;
   h.mats_off = o; o += a256(sizeof(BatchMat) * (size_t)count);
   h.item_mat_off = o; o += a256(4 * (size_t)items);
-  // arrival counts per (item, column tile), then the work counters: one
-  // memset per step clears both
+  h.tprobs_off = o; o += a256(sizeof(TileProb) * (size_t)h.tile_count);
+  h.titem_off = o; o += a256(4 * (size_t)titems);
+  // arrival counts per (item, column tile) and (tile, column phase), then the
+  // work counters: one memset per step clears them
   h.rows_off = o; o += 4 * (size_t)items * (size_t)(h.tiles > 0 ? h.tiles : 1);
+  h.tcnt_off = o; o += 4 * (size_t)titems * (size_t)h.tphases;
   h.counter_off = o; o = a256(o + 4 * (size_t)(h.tiles > 0 ? h.tiles : 1));
   h.heads_off = o; o += a256(4 * (size_t)items * N);
   h.tails_off = o; o += a256(4 * (size_t)items * N);
+  h.theads_off = o; o += a256(4 * (size_t)titems * N);
+  h.ttails_off = o; o += a256(4 * (size_t)titems * N);
   h.dev_bytes = o;
   // the walk stores head/tail partials as vectors of up to 32 bytes
   if ((h.heads_off | h.tails_off | h.mats_off | h.item_mat_off | h.rows_off) & 255)
@@ -93,7 +121,22 @@ static ss_status batch_layout(int count, const ss_csr *mats, int N, const ss_kno
 }
 
 static size_t host_bytes_for(const BatchHeader &h) {
-  return a256(sizeof(BatchHeader)) + a256(sizeof(BatchMat) * (size_t)h.count) + a256(4 * (size_t)h.total_items);
+  return a256(sizeof(BatchHeader)) + a256(sizeof(BatchMat) * (size_t)h.count) + a256(4 * (size_t)h.total_items) +
+         a256(sizeof(TileProb) * (size_t)h.tile_count) + a256(4 * (size_t)h.tile_items);
+}
+
+// The sizes a plan may need, whatever the alignment of its operands.
+static ss_status batch_most(int count, const ss_csr *mats, int N, const ss_knobs *per_mat, const int *strategies,
+                            size_t *host, size_t *dev) {
+  *host = *dev = 0;
+  for (int v = 1; v <= 8; v <<= 1) {
+    BatchHeader h;
+    ss_status st = batch_layout(count, mats, N, per_mat, strategies, v, h, nullptr, nullptr);
+    if (st) return st;
+    *host = std::max(*host, host_bytes_for(h));
+    *dev = std::max(*dev, h.dev_bytes);
+  }
+  return SS_OK;
 }
 
 }  // namespace ss
@@ -105,12 +148,7 @@ extern "C" {
 ss_status ss_batch_plan_size_ex(int count, const ss_csr *mats, int N, const ss_knobs *per_mat,
                                 const int *per_mat_strategy, size_t *host_bytes, size_t *dev_bytes) {
   if (!host_bytes || !dev_bytes) return fail(SS_ERR_INVALID_ARG, "null size pointer");
-  BatchHeader h;
-  ss_status st = batch_layout(count, mats, N, per_mat, per_mat_strategy, h, nullptr);
-  if (st) return st;
-  *host_bytes = host_bytes_for(h);
-  *dev_bytes = h.dev_bytes;
-  return SS_OK;
+  return batch_most(count, mats, N, per_mat, per_mat_strategy, host_bytes, dev_bytes);
 }
 
 ss_status ss_batch_plan_ex(int count, const ss_csr *mats, int N, const void *const *B, void *const *C,
@@ -119,7 +157,14 @@ ss_status ss_batch_plan_ex(int count, const ss_csr *mats, int N, const void *con
   if (!B || !C || !host_buf || !dev_buf) return fail(SS_ERR_INVALID_ARG, "null pointer");
   BatchHeader h;
   std::vector<BatchMat> bm;
-  ss_status st = batch_layout(count, mats, N, per_mat, per_mat_strategy, h, &bm);
+  std::vector<TileProb> tp;
+  if (count < 1 || !mats || N < 1) return fail(SS_ERR_INVALID_ARG, "batch needs count >= 1, N >= 1 and matrices");
+  if (mats[0].value_dtype < SS_F32 || mats[0].value_dtype > SS_F16 || c_dtype < SS_F32 || c_dtype > SS_F16)
+    return fail(SS_ERR_INVALID_ARG, "unknown dtype");
+  int vmax = 16 / dtype_size(mats[0].value_dtype);
+  for (int m = 0; m < count; m++)
+    vmax = std::min(vmax, tile_vmax(B[m], dtype_size(mats[0].value_dtype), C[m], dtype_size(c_dtype)));
+  ss_status st = batch_layout(count, mats, N, per_mat, per_mat_strategy, vmax, h, &bm, &tp);
   if (st) return st;
   if (c_dtype != SS_F32 && c_dtype != h.val_dtype) return fail(SS_ERR_INVALID_ARG, "c_dtype must be F32 or the value dtype");
   h.c_dtype = c_dtype;
@@ -142,11 +187,30 @@ ss_status ss_batch_plan_ex(int count, const ss_csr *mats, int N, const void *con
   int32_t *him = (int32_t *)((char *)hm + a256(sizeof(BatchMat) * (size_t)count));
   for (int m = 0; m < count; m++)
     for (int c = 0; c < bm[m].num_chunks; c++) him[bm[m].item_begin + c] = m;
+  TileProb *ht = (TileProb *)((char *)him + a256(4 * (size_t)h.total_items));
+  int32_t *hti = (int32_t *)((char *)ht + a256(sizeof(TileProb) * (size_t)h.tile_count));
+  char *db = (char *)dev_buf;
+  for (int i = 0; i < h.tile_count; i++) {
+    TileProb &p = tp[i];
+    const int m = p.index;
+    p.B = B[m];
+    p.C = C[m];
+    p.cnt = (int *)(db + h.tcnt_off) + (size_t)p.item_begin * h.tphases;
+    p.heads = (float *)(db + h.theads_off) + (size_t)p.item_begin * N;
+    p.tails = (float *)(db + h.ttails_off) + (size_t)p.item_begin * N;
+    const int end = i + 1 < h.tile_count ? tp[i + 1].item_begin : h.tile_items;
+    for (int c = p.item_begin; c < end; c++) hti[c] = i;
+  }
+  if (h.tile_count > 0) memcpy(ht, tp.data(), sizeof(TileProb) * (size_t)h.tile_count);
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaMemcpyAsync((char *)dev_buf + h.mats_off, hm, sizeof(BatchMat) * (size_t)count,
                                   cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && h.total_items > 0)
     e = cudaMemcpyAsync((char *)dev_buf + h.item_mat_off, him, 4 * (size_t)h.total_items, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && h.tile_count > 0)
+    e = cudaMemcpyAsync(db + h.tprobs_off, ht, sizeof(TileProb) * (size_t)h.tile_count, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && h.tile_items > 0)
+    e = cudaMemcpyAsync(db + h.titem_off, hti, 4 * (size_t)h.tile_items, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the host buffer may be reused after return
   return e == cudaSuccess ? SS_OK : cuda_fail(e, "batch plan upload");
 }
@@ -168,14 +232,35 @@ ss_status ss_spmm_batched(const void *host_plan, void *dev_plan, void *stream) {
   if (!host_plan || !dev_plan) return fail(SS_ERR_INVALID_ARG, "null plan");
   BatchHeader h;
   memcpy(&h, host_plan, sizeof(h));
-  if (h.total_items == 0) return SS_OK;
+  if (h.total_items == 0 && h.tile_items == 0) return SS_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  char *plan = (char *)dev_plan;
+  // arrival counts and work counters (adjacent in the plan)
+  cudaError_t e = cudaMemsetAsync(plan + h.rows_off, 0, h.heads_off - h.rows_off, s);
+  if (e != cudaSuccess) return cuda_fail(e, "batched counter reset");
+  if (h.tile_items > 0) {
+    TileArgs a;
+    memset(&a, 0, sizeof(a));
+    a.probs = (const TileProb *)(plan + h.tprobs_off);
+    a.item_prob = (const int32_t *)(plan + h.titem_off);
+    a.items = h.tile_items;
+    a.phases = h.tphases;
+    a.N = h.N;
+    a.kahan = h.kahan;
+    a.keep_frac = 1.0f;
+    TileGeom g;
+    memset(&g, 0, sizeof(g));
+    g.G = h.tG;
+    g.V = h.tV;
+    g.NV = h.tNV;
+    ss_status st = run_tile(h.val_dtype, h.c_dtype, g, h.tsmem, a, s);
+    if (st || h.total_items == 0) return st;
+  }
   void *fn;
   if (h.val_dtype == SS_F32) fn = batched_kernel_f32(h.V, h.NV);
   else if (h.val_dtype == SS_BF16) fn = batched_kernel_bf16(h.V, h.NV, h.c_dtype == SS_F32);
   else fn = batched_kernel_f16(h.V, h.NV, h.c_dtype == SS_F32);
   if (!fn) return fail(SS_ERR_UNSUPPORTED_KNOBS, "no batched kernel for V=%d NV=%d", h.V, h.NV);
-  cudaError_t e;
   if (h.smem > 48 * 1024) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.smem);
     if (e != cudaSuccess) return cuda_fail(e, "batched smem attribute");
@@ -186,11 +271,7 @@ ss_status ss_spmm_batched(const void *host_plan, void *dev_plan, void *stream) {
   long long grid = (long long)per_sm * sm_count();
   const long long need = ((long long)h.total_items + h.workers_per_block - 1) / h.workers_per_block;
   if (grid > need) grid = need;
-  // arrival counts and work counters (adjacent in the plan)
-  e = cudaMemsetAsync((char *)dev_plan + h.rows_off, 0, h.heads_off - h.rows_off, s);
-  if (e != cudaSuccess) return cuda_fail(e, "batched counter reset");
   int *err_ptr = walk_error_ptr();
-  const char *plan = (const char *)dev_plan;
   void *args[] = {&plan, &h, &err_ptr};
   e = cudaLaunchKernel(fn, dim3((unsigned)grid, (unsigned)h.tiles, 1), dim3(h.block, 1, 1), args, h.smem, s);
   return e == cudaSuccess ? SS_OK : cuda_fail(e, "batched launch");

@@ -2,19 +2,21 @@
 //
 // No counterpart in the reference (its drivers launch one matrix at a time).
 // A plan (host + device copies, built by ss_batch_plan) lists the matrices
-// and numbers their work items: item i is chunk (i - item_begin[m]) of
-// matrix m = item_mat[i], a chunk being thread_nz * G consecutive nonzeros
-// of that matrix (its own knob, element-balanced), or, for a matrix planned
-// row-balanced, a block of whole rows holding about that many nonzeros (each
-// row then summed in order by one group, as rbsr sums it).  The persistent kernel runs one resident
-// wave; every group takes the next item from a device counter (atomicAdd,
-// no waiting on other groups) and walks it with the ebsr chunk walk
-// (eb_walk.cuh) against that matrix's arrays.  Straddling rows go to the
-// matrix's head/tail slots and the last of their chunks to finish
-// assembles them (carry_arrive), so one launch does the whole step.
-// Matrices without nonzeros get a zero-fill item.  The whole step (counter
-// reset, walk) is stream-ordered and can be captured in a graph.
+// and numbers their work items.  Element-balanced matrices are walked by the
+// tile walk (eb_tile.cuh), one block per tile.  Matrices planned
+// row-balanced (items are blocks of whole rows holding about thread_nz * G
+// nonzeros, each row summed in order by one group, as rbsr sums it) and
+// matrices whose tuple asks for sequential runs of more than 2048 nonzeros
+// go to a persistent kernel: every group takes the next item from a device
+// counter (atomicAdd, no waiting on other groups) and walks it with the
+// ebsr chunk walk (eb_walk.cuh) against that matrix's arrays.  Straddling
+// rows go to the matrix's head/tail slots and the last of their tiles
+// or chunks to finish assembles them, so a step is one memset and one launch
+// (two when a batch has matrices of both kinds).
+// Matrices without nonzeros are an empty tile, whose block writes the zeros.
+// The whole step is stream-ordered and can be captured in a graph.
 #pragma once
+#include "eb_tile.cuh"
 #include "eb_walk.cuh"
 
 namespace ss {
@@ -27,7 +29,7 @@ struct BatchMat {
   void *C;
   int M, K, nnz;
   int chunk;          // element-balanced: nonzeros per item
-  int num_chunks;     // items of this matrix (1 zero-fill item when nnz == 0)
+  int num_chunks;     // items of this matrix in the persistent kernel (0: walked by tiles)
   int item_begin;     // first item of this matrix
   int use_tma;
   int rows_per_item;  // row-balanced (> 0): whole rows per item, no row split
@@ -40,6 +42,9 @@ struct BatchHeader {
   // device-side offsets (bytes from the plan base)
   size_t mats_off, item_mat_off, rows_off, heads_off, tails_off, counter_off;
   size_t dev_bytes;
+  // matrices walked by tiles
+  int tile_count, tile_items, tG, tV, tNV, tphases;
+  size_t tsmem, tprobs_off, titem_off, tcnt_off, tstarts_off, theads_off, ttails_off;
 };
 
 template <typename T, typename TC, int V, int NV>
@@ -104,12 +109,6 @@ __global__ void __launch_bounds__(512, SS_SR_MIN_BLOCKS) batched_kernel(const ch
     const int m = item_mat[item];
     const BatchMat mt = mats[m];
     const int chunk = item - mt.item_begin;
-    if (mt.nnz == 0) {  // zero-fill item
-      a.M = mt.M;
-      a.C = mt.C;
-      zero_rows<TC, V, NV>(a, 0, mt.M - 1, col0, act, strm);
-      continue;
-    }
     a.M = mt.M;
     a.K = mt.K;
     a.nnz = mt.nnz;

@@ -340,11 +340,15 @@ __device__ __forceinline__ void kahan_add(float &acc, float &c, float x) {
   acc = t;
 }
 
-// acc += v * b with compensation.  The product is rounded on its own
-// (__fmul_rn is never contracted into an FMA with the step that follows), so
-// every kernel that sums the same terms in the same order gets the same bits.
+// acc += v * b with compensation: the product enters the corrected term
+// unrounded.  Every operation is spelled out, so no kernel's contraction
+// differs and the kernels that sum the same terms in the same order get the
+// same bits.
 __device__ __forceinline__ void kahan_fma(float &acc, float &c, float v, float b) {
-  kahan_add(acc, c, __fmul_rn(v, b));
+  const float y = __fmaf_rn(v, b, -c);
+  const float t = __fadd_rn(acc, y);
+  c = __fsub_rn(__fsub_rn(t, acc), y);
+  acc = t;
 }
 
 // Lane mask of the aligned sub-warp of `width` lanes containing this lane.

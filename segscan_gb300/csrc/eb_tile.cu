@@ -1,0 +1,142 @@
+// Geometry and launch of the tile walk (kernel in eb_tile.cuh).
+#include <algorithm>
+#include <cstring>
+
+#include "eb_tile.cuh"
+
+namespace ss {
+
+// row_start[t] = first row that starts at or after nonzero t * tile_nz
+// (row_start[tiles] = M), one thread per row; also clears the arrival
+// counts, so the walk needs no memset of its own.  2 us on a million rows,
+// against 2.5 us of search latency in every block of the walk (N = 64:
+// 207 -> 203 us).
+__global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restrict__ indptr, int M, int log2_tile,
+                                                        int tiles, int32_t *__restrict__ row_start,
+                                                        int *__restrict__ cnt, int ncnt) {
+  const long long stride = (long long)gridDim.x * 256, i0 = blockIdx.x * 256ll + threadIdx.x;
+  for (long long r0 = i0 * 4; r0 <= M; r0 += stride * 4) {
+    int x[5];
+    x[0] = r0 > 0 ? __ldg(indptr + r0 - 1) >> log2_tile : -1;
+    #pragma unroll
+    for (int i = 0; i < 4; i++) x[i + 1] = r0 + i <= M ? __ldg(indptr + r0 + i) >> log2_tile : INT_MIN;
+    #pragma unroll
+    for (int i = 0; i < 4; i++)
+      for (int t = max(x[i] + 1, 0); t <= min(x[i + 1], tiles - 1); t++) row_start[t] = (int)r0 + i;
+  }
+  if (i0 == 0) row_start[tiles] = M;
+  for (long long i = i0; i < ncnt; i += stride) cnt[i] = 0;
+}
+
+TileGeom tile_geom(int N, int nnz, int dtype, int vmax) {
+  TileGeom g;
+  int V = std::min(16 / dtype_size(dtype), std::max(1, vmax));
+  while (N % V) V >>= 1;
+  const int nv = ceil_div(N, V);
+  g.V = V;
+  g.NV = 1;
+  g.G = std::min(16, ceil_pow2(nv));
+  // widths that no wide vector divides: several vectors per lane, as many as
+  // leave the fewest idle columns (N = 47: 16 lanes of three, 108 us, against
+  // three phases of one, 252 us)
+  const int most = V == 1 ? 4 : V == 2 ? 2 : 1;
+  if (nv > 16)
+    for (int m = 2; m <= most; m++)
+      if (ceil_div(nv, 16 * m) * m <= ceil_div(nv, 16 * g.NV) * g.NV) g.NV = m;
+  g.phases = ceil_div(N, g.G * V * g.NV);
+  // pieces as long as shared memory allows without costing resident blocks
+  // (2048 nonzeros a tile, 1024 with 16 lanes), shorter where a matrix would
+  // otherwise fill less than two blocks per SM
+  const int NG = TW_T / g.G;
+  int slog = g.G >= 16 ? 6 : 3 + ilog2(g.G);
+  while (slog > 3 && (long long)nnz < ((long long)NG << slog) * 2 * sm_count()) slog--;
+  g.slog = slog;
+  g.tile = NG << slog;
+  g.tiles = std::max(1, ceil_div(nnz, g.tile));
+  g.smem = (size_t)tile_smem(g.G, V * g.NV, slog).total * 4;
+  return g;
+}
+
+// The tile walk's scratch grows with the matrix (two partial rows a tile), the
+// group walk's does not: past 2^18 tiles (256 M nonzeros at 16 lanes, 128 MB
+// at N = 64) the group walk keeps it.  It also takes what a block index or a
+// 32-bit row stride cannot hold.
+bool tile_fits(int N, int nnz, int dtype) {
+  if (N >= (1 << 29)) return false;
+  for (int v = 1; v <= 16 / dtype_size(dtype); v <<= 1) {
+    const TileGeom g = tile_geom(N, nnz, dtype, v);
+    if (g.tiles > 1 << 18 || (long long)g.tiles * g.phases >= (1LL << 31)) return false;
+  }
+  return true;
+}
+
+static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+static size_t tile_ws(const TileGeom &g, int N) {
+  return align256((size_t)g.tiles * g.phases * 4) + align256((size_t)(g.tiles + 1) * 4) +
+         2 * (size_t)g.tiles * (size_t)N * sizeof(float);
+}
+
+size_t tile_workspace_bytes(int N, int nnz, int dtype) {
+  // the alignment of B and C, and so the vector, is not known to the query
+  size_t most = 0;
+  for (int v = 1; v <= 16 / dtype_size(dtype); v <<= 1) most = std::max(most, tile_ws(tile_geom(N, nnz, dtype, v), N));
+  return most;
+}
+
+int tile_vmax(const void *B, int b_bytes, const void *C, int c_bytes) {
+  int v = 16 / b_bytes;
+  while (v > 1 && (((uintptr_t)B % (size_t)(b_bytes * v)) || ((uintptr_t)C % (size_t)std::min(16, c_bytes * v)))) v >>= 1;
+  return v;
+}
+
+static void *tile_kernel(int val_dtype, int c_dtype, int G, int V, int NV, bool addc) {
+  if (val_dtype == SS_F32)
+    return c_dtype == SS_F32    ? tile_kernel_f32(G, V, NV, addc)
+           : c_dtype == SS_BF16 ? tile_kernel_f32_bf16(G, V, NV, addc)
+                                : tile_kernel_f32_f16(G, V, NV, addc);
+  if (val_dtype == SS_BF16) return c_dtype == SS_F32 ? tile_kernel_bf16_f32(G, V, NV, addc) : tile_kernel_bf16(G, V, NV, addc);
+  return c_dtype == SS_F32 ? tile_kernel_f16_f32(G, V, NV, addc) : tile_kernel_f16(G, V, NV, addc);
+}
+
+ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, cudaStream_t s) {
+  void *fn = tile_kernel(val_dtype, c_dtype, g.G, g.V, g.NV, a.accumulate != 0);
+  if (!fn) return fail(SS_ERR_UNSUPPORTED_KNOBS, "no tile walk for G=%d V=%d NV=%d", g.G, g.V, g.NV);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "tile walk shared memory");
+  }
+  void *args[] = {&a};
+  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)(a.items * a.phases), 1, 1), dim3(TW_T, 1, 1), args, smem, s);
+  return e == cudaSuccess ? SS_OK : cuda_fail(e, "tile walk launch");
+}
+
+ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
+  const TileGeom g = tile_geom(c.N, c.nnz, c.val_dtype,
+                               tile_vmax(c.B, dtype_size(c.val_dtype), c.C, dtype_size(c.c_dtype)));
+  TileArgs a;
+  memset(&a, 0, sizeof(a));
+  TileProb &p = a.p;
+  p.indptr = c.indptr; p.cols = c.indices; p.vals = c.vals; p.B = c.B; p.C = c.C;
+  p.M = c.M; p.K = c.K; p.nnz = c.nnz;
+  p.slog = g.slog;
+  p.wide = (((uintptr_t)c.indices | (uintptr_t)c.vals) & 15u) == 0;
+  char *w = (char *)ws;
+  p.cnt = (int *)w; w += align256((size_t)g.tiles * g.phases * 4);
+  int32_t *row_start = (int32_t *)w; w += align256((size_t)(g.tiles + 1) * 4);
+  p.row_start = row_start;
+  p.heads = (float *)w;
+  p.tails = p.heads + (size_t)g.tiles * c.N;
+  a.items = g.tiles; a.phases = g.phases;
+  a.N = c.N; a.accumulate = c.accumulate; a.kahan = c.kahan_threshold;
+  a.keep_frac = l2_keep_fraction((size_t)c.K * c.N * dtype_size(c.val_dtype));
+  const int ncnt = g.tiles * g.phases;
+  const long long want = ((long long)c.M + 1024) / 1024;
+  tile_rows_kernel<<<(unsigned)std::min(want, (long long)sm_count() * 16), 256, 0, s>>>(c.indptr, c.M, ilog2(g.tile), g.tiles,
+                                                                                      row_start, p.cnt, ncnt);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "tile rows launch");
+  return run_tile(c.val_dtype, c.c_dtype, g, g.smem, a, s);
+}
+
+}  // namespace ss

@@ -1,0 +1,613 @@
+// Element-balanced SpMM over block tiles: the ebsr walk of one matrix and of
+// the batched launch.
+//
+// Reference counterpart: csrspmm_rowcaching_nnzbalance_cg_kernel
+// (test-cg/include/spmm/spmm_cg.cuh:376-551).
+//
+// A block takes a tile of consecutive nonzeros, cut into equal pieces, one
+// per group of G lanes laid along N (E = V * NV columns a
+// lane), and
+//  * the tile's columns and values go to shared memory with plain 16-byte
+//    loads, each piece padded by four words so that the groups of a warp
+//    read their streams without bank conflicts;
+//  * the rows that start in the tile (row_start, or a warp search) mark their
+//    last nonzero with row + 1 and write the empty rows; no nonzero is
+//    searched or labelled one by one;
+//  * a group walks its piece four nonzeros at a time: four B rows gathered
+//    together, four multiply-adds, and at a marked nonzero the finished row
+//    is stored by a predicated store, so groups of one warp do not diverge
+//    at their row ends;
+//  * a group's first row end may belong to a row that an earlier group
+//    started: it goes to shared memory with every group's last partial, and
+//    the pieces of a row are added in order after the walk;
+//  * rows that straddle tiles go through one head and one tail slot per tile
+//    and the last participant stores them (tile_arrive), as in carry_arrive.
+// Nonzeros of rows longer than kahan_threshold are summed with compensation:
+// warps that hold any take a second instantiation of the walk, which also
+// skips columns outside [0, K).
+//
+// What bounds it (power-law 1e6 x 1e6, 4.6 M nonzeros): at N = 64 FP32 the
+// gathered rows, 1.13 GB of DRAM traffic at 5.5 TB/s; with 16-bit storage
+// and at small N the issue of about 35 instructions per gathered vector.
+#pragma once
+
+#include "eb_common.cuh"
+#include "internal.h"
+
+namespace ss {
+
+constexpr int TW_T = 256;  // threads per block
+
+// One matrix of a launch (16-byte multiple: copied by 16-byte words).
+struct __align__(16) TileProb {
+  const int32_t *indptr, *cols;
+  const void *vals;  // null = ones
+  const void *B;
+  void *C;
+  const int32_t *row_start;  // [tiles + 1] first row starting at or after each tile, or null: searched
+  int *cnt;                  // [tiles * phases] arrivals per straddling row
+  float *heads, *tails;      // [tiles * N] partials of a tile's first / last row
+  int M, K, nnz;
+  int slog;        // a piece is 1 << slog nonzeros
+  int item_begin;  // first block of this matrix (batched)
+  int wide;        // columns and values may be loaded 16 bytes at a time
+  int index;       // host: the matrix's place in its batch
+  int pad;
+};
+
+struct TileArgs {
+  TileProb p;              // the matrix (single launch)
+  const TileProb *probs;   // batched: the matrices ...
+  const int32_t *item_prob;  // ... and the matrix of each block; null = single
+  int items, phases;       // blocks per column phase
+  int N, accumulate, kahan;
+  float keep_frac;
+};
+
+// Shared memory of a block, in words after the TileProb.
+struct TileSmem {
+  int col, val, info, head, tail, kb, ends, total;
+};
+__host__ __device__ inline TileSmem tile_smem(int G, int E, int slog) {
+  const int NG = TW_T / G, words = NG * ((1 << slog) + 4);
+  TileSmem s;
+  int o = (int)sizeof(TileProb) / 4;
+  s.col = o; o += words;
+  s.val = o; o += words;
+  s.info = o; o += words;
+  s.head = o; o += TW_T * E;
+  s.tail = o; o += TW_T * E;
+  s.kb = o; o += ((NG << slog) + 31) / 32;
+  s.ends = o; o += (NG + 31) / 32;
+  s.total = o;
+  return s;
+}
+
+template <int V>
+__device__ __forceinline__ void store_smem(float *p, const float (&v)[V]) {
+  if constexpr (V % 4 == 0) {
+    #pragma unroll
+    for (int i = 0; i < V; i += 4)
+      *reinterpret_cast<float4 *>(p + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+  } else if constexpr (V == 2) {
+    *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+  } else {
+    p[0] = v[0];
+  }
+}
+
+// V elements of the output, widened (plain loads: the row is rewritten here).
+template <typename TC, int V>
+__device__ __forceinline__ void load_old(const TC *p, float (&out)[V]) {
+  if constexpr (V * sizeof(TC) > 16) {
+    constexpr int H = V / 2;
+    float lo[H], hi[H];
+    load_old<TC, H>(p, lo);
+    load_old<TC, H>(p + H, hi);
+    #pragma unroll
+    for (int i = 0; i < H; i++) { out[i] = lo[i]; out[H + i] = hi[i]; }
+  } else {
+    RawVec<TC, V> r;
+    if constexpr (V * sizeof(TC) == 16) {
+      const uint4 x = *reinterpret_cast<const uint4 *>(p);
+      r.w[0] = x.x; r.w[1] = x.y; r.w[2] = x.z; r.w[3] = x.w;
+    } else if constexpr (V * sizeof(TC) == 8) {
+      const uint2 x = *reinterpret_cast<const uint2 *>(p);
+      r.w[0] = x.x; r.w[1] = x.y;
+    } else if constexpr (V * sizeof(TC) == 4) {
+      r.w[0] = *reinterpret_cast<const uint32_t *>(p);
+    } else {
+      r.w[0] = *reinterpret_cast<const uint16_t *>(p);
+    }
+    unpack_raw<TC, V>(r, out);
+  }
+}
+
+// One predicated instruction each, so that groups of one warp do not branch
+// apart where only some of them end a row.
+__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[4], uint64_t pol, bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %6, 0;\n"
+               " @p st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %5;\n}" ::"l"(p), "r"(w[0]), "r"(w[1]),
+               "r"(w[2]), "r"(w[3]), "l"(pol), "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[2], uint64_t pol, bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+               " @p st.global.L2::cache_hint.v2.u32 [%0], {%1, %2}, %3;\n}" ::"l"(p), "r"(w[0]), "r"(w[1]), "l"(pol),
+               "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[1], uint64_t pol, bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.global.L2::cache_hint.u32 [%0], %1, %2;\n}" ::
+               "l"(p), "r"(w[0]), "l"(pol), "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void st16_if(void *p, uint16_t w, uint64_t pol, bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.global.L2::cache_hint.u16 [%0], %1, %2;\n}" ::
+               "l"(p), "h"(w), "l"(pol), "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[4], bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n @p ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n}"
+               : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]) : "l"(p), "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[2], bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p ld.global.v2.u32 {%0, %1}, [%2];\n}"
+               : "+r"(w[0]), "+r"(w[1]) : "l"(p), "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[1], bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.global.u32 %0, [%1];\n}"
+               : "+r"(w[0]) : "l"(p), "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void ld16_if(const void *p, uint32_t &w, bool on) {
+  uint16_t h = 0;
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.global.u16 %0, [%1];\n}"
+               : "+h"(h) : "l"(p), "r"((unsigned)on) : "memory");
+  w = h;
+}
+template <typename T, int V>
+__device__ __forceinline__ void store_vec_if(T *p, const float (&v)[V], uint64_t pol, bool on) {
+  if constexpr (V * sizeof(T) > 16) {
+    constexpr int H = V / 2;
+    float lo[H], hi[H];
+    #pragma unroll
+    for (int i = 0; i < H; i++) { lo[i] = v[i]; hi[i] = v[H + i]; }
+    store_vec_if<T, H>(p, lo, pol, on);
+    store_vec_if<T, H>(p + H, hi, pol, on);
+  } else if constexpr (V * sizeof(T) == 2) {
+    const T h = Elem<T>::from_f(v[0]);
+    st16_if(p, *reinterpret_cast<const uint16_t *>(&h), pol, on);
+  } else {
+    uint32_t w[V * sizeof(T) / 4];
+    #pragma unroll
+    for (int i = 0; i < (int)(V * sizeof(T) / 4); i++) {
+      if constexpr (sizeof(T) == 4) w[i] = __float_as_uint(v[i]);
+      else w[i] = pack2(v[2 * i], v[2 * i + 1], (T *)nullptr);
+    }
+    st_if(p, w, pol, on);
+  }
+}
+// V elements of the output as words, kept packed until they are added.
+template <typename T, int V>
+struct OldVec {
+  static constexpr int B = V * (int)sizeof(T), W = B > 16 ? 4 : (B + 3) / 4, P = (B + 15) / 16;
+  uint32_t w[P][W];
+};
+template <typename T, int V>
+__device__ __forceinline__ void load_old_if(const T *p, OldVec<T, V> &o, bool on) {
+  #pragma unroll
+  for (int k = 0; k < OldVec<T, V>::P; k++) {
+    const char *q = (const char *)p + 16 * k;
+    if constexpr (OldVec<T, V>::B == 2) ld16_if(q, o.w[k][0], on);
+    else ld_if(q, o.w[k], on);
+  }
+}
+template <typename T, int V>
+__device__ __forceinline__ void unpack_old(const OldVec<T, V> &o, float (&out)[V]) {
+  constexpr int VP = V / OldVec<T, V>::P;
+  #pragma unroll
+  for (int k = 0; k < OldVec<T, V>::P; k++) {
+    RawVec<T, VP> r;
+    float x[VP];
+    #pragma unroll
+    for (int i = 0; i < OldVec<T, V>::W; i++) r.w[i] = o.w[k][i];
+    unpack_raw<T, VP>(r, x);
+    #pragma unroll
+    for (int i = 0; i < VP; i++) out[k * VP + i] = x[i];
+  }
+}
+
+template <int V, int NV>
+__device__ __forceinline__ void clear(float (&x)[NV][V]) {
+  #pragma unroll
+  for (int j = 0; j < NV; j++)
+    #pragma unroll
+    for (int i = 0; i < V; i++) x[j][i] = 0.f;
+}
+
+// Row `row` of C = acc (+ the old row in accumulate mode), this lane's columns.
+template <typename TC, int G, int V, int NV, bool ADDC>
+__device__ __forceinline__ void tile_store(const TileProb &p, int N, int row, const float (&acc)[NV][V],
+                                           int col0, const bool (&act)[NV], uint64_t pol) {
+  if ((unsigned)row >= (unsigned)p.M) return;
+  TC *dst = (TC *)p.C + (int64_t)row * N + col0;
+  #pragma unroll
+  for (int j = 0; j < NV; j++) {
+    if (!act[j]) continue;
+    TC *d = dst + j * G * V;
+    float x[V];
+    #pragma unroll
+    for (int i = 0; i < V; i++) x[i] = acc[j][i];
+    if (ADDC) {
+      float prev[V];
+      load_old<TC, V>(d, prev);
+      #pragma unroll
+      for (int i = 0; i < V; i++) x[i] += prev[i];
+    }
+    store_vec<TC, V>(d, x, pol);
+  }
+}
+
+// Counts this tile in for row r, which straddles tiles o..l; the last tile to
+// arrive sums tail(o) + heads(o+1..l) in tile order with compensation and
+// stores the row, so the result does not depend on which one is last.
+template <typename TC, int G, int V, int NV, bool ADDC>
+__device__ __forceinline__ void tile_arrive(const TileProb &p, int N, int tile_nz, int r, int lane,
+                                            unsigned mask, int phase, int phases, int col0, const bool (&act)[NV],
+                                            uint64_t pol) {
+  const int s = __ldg(p.indptr + r), e = __ldg(p.indptr + r + 1);
+  if ((unsigned)s >= (unsigned)p.nnz || (unsigned)(e - 1) >= (unsigned)p.nnz) return;  // malformed indptr
+  const int o = s / tile_nz, l = (e - 1) / tile_nz;
+  __threadfence();  // this lane's slot stores are visible before the count moves
+  __syncwarp(mask);
+  int last = 0;
+  if (lane == 0) last = atomicAdd(p.cnt + (size_t)o * phases + phase, 1) == l - o;
+  last = __shfl_sync(mask, last, 0, G);
+  if (!last) return;
+  __threadfence();  // every other participant's slot is visible now
+  float acc[NV][V];
+  clear<V, NV>(acc);
+  #pragma unroll
+  for (int j = 0; j < NV; j++) {
+    if (!act[j]) continue;
+    const int64_t col = col0 + j * G * V;
+    float comp[V], x[V];
+    load_slot<V>(p.tails + (int64_t)o * N + col, acc[j]);
+    #pragma unroll
+    for (int i = 0; i < V; i++) comp[i] = 0.f;
+    for (int k = o + 1; k <= l; k++) {
+      load_slot<V>(p.heads + (int64_t)k * N + col, x);
+      #pragma unroll
+      for (int i = 0; i < V; i++) kahan_add(acc[j][i], comp[i], x[i]);
+    }
+  }
+  tile_store<TC, G, V, NV, ADDC>(p, N, r, acc, col0, act, pol);
+}
+
+// One group's piece: S nonzeros from its staged columns, values and row-end
+// marks.  The first row end goes to shead (its row + 1 is returned, 0 when
+// the piece has none), what follows the last one to stail, the others to C.
+template <typename T, typename TC, int G, int V, int NV, bool SLOW, bool ADDC>
+__device__ __forceinline__ int tile_walk(const TileProb &p, int N, int S, const int32_t *scol,
+                                         const float *sval, const int32_t *sinfo, const uint32_t *kb, int p0,
+                                         float *shead, float *stail, int lane, int col0, const bool (&act)[NV],
+                                         uint64_t keep, uint64_t strm) {
+  const char *Bj[NV];
+  char *Cj[NV];
+  const uint32_t ldb = (uint32_t)N * (uint32_t)sizeof(T), ldc = (uint32_t)N * (uint32_t)sizeof(TC);
+  #pragma unroll
+  for (int j = 0; j < NV; j++) {
+    // a lane past the last column repeats a column that it (or lane 0)
+    // computes too and stores the same value to the same place: no predicate
+    // per load and store
+    const int cj = act[j] ? col0 + j * G * V : act[0] ? col0 : col0 - lane * V;
+    Bj[j] = (const char *)((const T *)p.B + cj);
+    Cj[j] = (char *)((TC *)p.C + cj) - ldc;  // marks hold row + 1
+  }
+  float acc[NV][V], comp[NV][V];
+  clear<V, NV>(acc);
+  clear<V, NV>(comp);
+  int hr = 0;
+  RawVec<T, V> raw[4][NV];
+  // accumulating: the rows of C that end among the four nonzeros, loaded with
+  // their B rows so that a row end does not wait for memory
+  OldVec<TC, V> old[ADDC ? 4 : 1][NV];
+  auto fetch = [&](int u, int c) {
+    #pragma unroll
+    for (int j = 0; j < NV; j++) {
+      if (!SLOW || c >= 0) load_raw<T, V>((const T *)(Bj[j] + (uint64_t)(uint32_t)c * ldb), raw[u][j], keep);
+      else zero_raw<T, V>(raw[u][j]);
+    }
+  };
+  auto consume = [&](int u, float v, int end, bool kah) {
+    #pragma unroll
+    for (int j = 0; j < NV; j++) {
+      float b[V];
+      unpack_raw<T, V>(raw[u][j], b);
+      if (SLOW && kah) {
+        #pragma unroll
+        for (int i = 0; i < V; i++) kahan_fma(acc[j][i], comp[j][i], v, b[i]);
+      } else {
+        #pragma unroll
+        for (int i = 0; i < V; i++) acc[j][i] = fmaf(v, b[i], acc[j][i]);
+      }
+    }
+    const bool first = end != 0 && hr == 0;
+    const bool out = end != 0 && hr != 0;
+    #pragma unroll
+    for (int j = 0; j < NV; j++) {
+      if (first) store_smem<V>(shead + j * G * V, acc[j]);
+      TC *d = (TC *)(Cj[j] + (uint64_t)(uint32_t)end * ldc);
+      if (ADDC) {
+        float x[V];
+        unpack_old<TC, V>(old[u][j], x);
+        #pragma unroll
+        for (int i = 0; i < V; i++) x[i] += acc[j][i];
+        store_vec_if<TC, V>(d, x, strm, out);
+      } else {
+        store_vec_if<TC, V>(d, acc[j], strm, out);
+      }
+      #pragma unroll
+      for (int i = 0; i < V; i++) {
+        acc[j][i] = end ? 0.f : acc[j][i];
+        if (SLOW) comp[j][i] = end ? 0.f : comp[j][i];
+      }
+    }
+    hr = first ? end : hr;
+  };
+  #pragma unroll 1
+  for (int q = 0; q < S; q += 4) {
+    const int4 c4 = *reinterpret_cast<const int4 *>(scol + q);
+    fetch(0, c4.x); fetch(1, c4.y); fetch(2, c4.z); fetch(3, c4.w);
+    const float4 v4 = *reinterpret_cast<const float4 *>(sval + q);
+    const int4 i4 = *reinterpret_cast<const int4 *>(sinfo + q);
+    if constexpr (ADDC) {
+      const int is[4] = {i4.x, i4.y, i4.z, i4.w};
+      #pragma unroll
+      for (int u = 0; u < 4; u++)
+        #pragma unroll
+        for (int j = 0; j < NV; j++)
+          load_old_if<TC, V>((const TC *)(Cj[j] + (uint64_t)(uint32_t)is[u] * ldc), old[u][j], is[u] != 0);
+    }
+    const uint32_t k4 = SLOW ? kb[(p0 + q) >> 5] >> ((p0 + q) & 31) : 0u;
+    consume(0, v4.x, i4.x, k4 & 1u);
+    consume(1, v4.y, i4.y, k4 & 2u);
+    consume(2, v4.z, i4.z, k4 & 4u);
+    consume(3, v4.w, i4.w, k4 & 8u);
+  }
+  #pragma unroll
+  for (int j = 0; j < NV; j++) store_smem<V>(stail + j * G * V, acc[j]);
+  return hr;
+}
+
+// Blocks per SM the registers are bounded for.  Five (48 registers) where a
+// lane holds one FP32 vector and the gathered rows are long (N = 64: 208 us
+// against 214 at four); at small N and with wider lanes the bound costs more
+// in spills than the fifth block gives (N = 4: 61 us at four, 74 at five;
+// BF16 N = 64: 157 and 225).  Accumulating needs four old rows beside the
+// gathered ones.
+template <typename T, int G, int V, int NV, bool ADDC>
+constexpr int tile_min_blocks() {
+  return ADDC ? (V * NV > 4 ? 2 : 3) : sizeof(T) == 4 && V == 4 && G >= 8 ? 5 : 4;
+}
+
+template <typename T, typename TC, int G, int V, int NV, bool ADDC>
+__global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) eb_tile_kernel(TileArgs a) {
+  constexpr int NG = TW_T / G, E = V * NV, COLS = G * E, EW = (NG + 31) / 32;
+  extern __shared__ __align__(16) int32_t smem[];
+  const int tid = threadIdx.x, wl = tid & 31;
+  const int phase = blockIdx.x / a.items;
+  const int item = blockIdx.x - phase * a.items;
+  if (tid < (int)sizeof(TileProb) / 16) {
+    const TileProb *src = a.item_prob ? a.probs + __ldg(a.item_prob + item) : &a.p;
+    reinterpret_cast<int4 *>(smem)[tid] = reinterpret_cast<const int4 *>(src)[tid];
+  }
+  __syncthreads();
+  const TileProb &p = *reinterpret_cast<const TileProb *>(smem);
+  const int S = 1 << p.slog, TILE = NG << p.slog;
+  const TileSmem L = tile_smem(G, E, p.slog);
+  int32_t *s_col = smem + L.col, *s_info = smem + L.info;
+  float *s_val = (float *)(smem + L.val), *s_head = (float *)(smem + L.head), *s_tail = (float *)(smem + L.tail);
+  uint32_t *s_kb = (uint32_t *)(smem + L.kb), *s_ends = (uint32_t *)(smem + L.ends);
+  __shared__ int s_rows[2];
+  const int tile = item - p.item_begin;
+  const uint64_t keep = policy_keep(a.keep_frac), strm = policy_stream();
+  const int lane = tid & (G - 1), g = tid / G;
+  const unsigned mask = G >= 32 ? 0xffffffffu : (((1u << (G & 31)) - 1u) << (wl & ~(G - 1)));
+  const int col0 = phase * COLS + lane * V;
+  bool act[NV];
+  #pragma unroll
+  for (int j = 0; j < NV; j++) act[j] = col0 + j * G * V < a.N;
+
+  const int ts = tile * TILE;
+  const int n = min(TILE, p.nnz - ts), te = ts + n;
+  // rows that start in the tile: [rlo, rhi)
+  int rlo, rhi;
+  if (p.row_start) {
+    rlo = __ldg(p.row_start + tile);
+    rhi = __ldg(p.row_start + tile + 1);
+  } else if (tid < 64) {
+    const int key = tid < 32 ? ts : te;
+    const int r = tid < 32 ? (ts == 0 ? 0 : group_lower_bound(p.indptr, p.M, key, wl, 32, 0xffffffffu))
+                           : (te >= p.nnz ? p.M : group_lower_bound(p.indptr, p.M, key, wl, 32, 0xffffffffu));
+    if (wl == 0) s_rows[tid >> 5] = r;
+  }
+  bool slow = false;
+  for (int e = tid * 4; e < TILE; e += TW_T * 4) {
+    int c[4];
+    float v[4] = {1.f, 1.f, 1.f, 1.f};
+    if (p.wide && e + 4 <= n) {
+      const uint4 x = ld_u128(p.cols + ts + e, strm);
+      c[0] = x.x; c[1] = x.y; c[2] = x.z; c[3] = x.w;
+      if (p.vals) load_vec<T, 4>((const T *)p.vals + ts + e, v, strm);
+    } else {
+      #pragma unroll
+      for (int i = 0; i < 4; i++) {
+        c[i] = e + i < n ? ld_idx(p.cols + ts + e + i, strm) : -1;
+        if (p.vals) v[i] = e + i < n ? load_val<T>((const T *)p.vals, (int64_t)ts + e + i, strm) : 0.f;
+      }
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; i++)
+      if ((unsigned)c[i] >= (unsigned)p.K) {
+        c[i] = -1;
+        slow = true;
+      }
+    const int w = e + 4 * (e >> p.slog);
+    *reinterpret_cast<int4 *>(s_col + w) = make_int4(c[0], c[1], c[2], c[3]);
+    *reinterpret_cast<float4 *>(s_val + w) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<int4 *>(s_info + w) = make_int4(0, 0, 0, 0);
+  }
+  for (int i = tid; i < (TILE + 31) / 32; i += TW_T) s_kb[i] = 0;
+  if (tid < EW) s_ends[tid] = 0;
+  if (!p.row_start) {
+    __syncthreads();
+    rlo = s_rows[0];
+    rhi = s_rows[1];
+  }
+  rlo = min(max(rlo, 0), p.M);
+  rhi = min(max(rhi, 0), p.M);
+  const bool has_head = rlo > 0 && __ldg(p.indptr + rlo) > ts;
+  const int rb = rlo - (has_head ? 1 : 0);
+  int rs = 0, re = 0;
+  if (rb + tid < rhi) {
+    rs = __ldg(p.indptr + rb + tid);
+    re = __ldg(p.indptr + rb + tid + 1);
+  }
+  __syncthreads();
+  // each row that ends in the tile marks its last nonzero; rows above the
+  // threshold mark all of theirs; empty rows are written here
+  for (int r0 = rb; r0 < rhi; r0 += TW_T) {
+    const int r = r0 + tid;
+    bool empty = false;
+    if (r < rhi) {
+      const int s = rs, e = re;
+      if (r + TW_T < rhi) {
+        rs = __ldg(p.indptr + r + TW_T);
+        re = __ldg(p.indptr + r + TW_T + 1);
+      }
+      empty = s == e;
+      const unsigned pos = (unsigned)(e - 1 - ts);
+      if (!empty && pos < (unsigned)n) s_info[pos + 4 * (pos >> p.slog)] = r + 1;
+      if (e - s > a.kahan) {
+        const int k0 = max(s - ts, 0), k1 = min(e - ts, n) - 1;
+        for (int w = k0 >> 5; w <= k1 >> 5; w++) {
+          uint32_t m = 0xffffffffu;
+          if (w == (k0 >> 5)) m &= 0xffffffffu << (k0 & 31);
+          if (w == (k1 >> 5)) m &= 0xffffffffu >> (31 - (k1 & 31));
+          atomicOr(s_kb + w, m);
+        }
+      }
+    }
+    if (!ADDC) {
+      unsigned todo = __ballot_sync(0xffffffffu, empty);
+      while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        if (wl < G) {
+          float z[NV][V];
+          clear<V, NV>(z);
+          tile_store<TC, G, V, NV, false>(p, a.N, r0 + (tid & ~31) + src, z, col0, act, strm);
+        }
+      }
+    }
+  }
+  slow = __syncthreads_or(slow);
+  {
+    const int WN = (32 / G) << p.slog, w0 = (tid >> 5) * WN;  // the warp's nonzeros
+    for (int w = w0 >> 5; w <= (w0 + WN - 1) >> 5; w++) slow |= s_kb[w] != 0;
+  }
+  const int gb = g * (S + 4);
+  float *shead = s_head + g * COLS + lane * V, *stail = s_tail + g * COLS + lane * V;
+  int hr;
+  if (!slow)
+    hr = tile_walk<T, TC, G, V, NV, false, ADDC>(p, a.N, S, s_col + gb, s_val + gb, s_info + gb, s_kb, g * S, shead,
+                                           stail, lane, col0, act, keep, strm);
+  else
+    hr = tile_walk<T, TC, G, V, NV, true, ADDC>(p, a.N, S, s_col + gb, s_val + gb, s_info + gb, s_kb, g * S, shead,
+                                          stail, lane, col0, act, keep, strm);
+  if (lane == 0 && hr) atomicOr(s_ends + (g >> 5), 1u << (g & 31));
+  __syncthreads();
+  // the last group before x with a row end, or -1
+  auto prev_end = [&](int x) {
+    int w = x >> 5;
+    uint32_t m = w < EW ? s_ends[w] & ((1u << (x & 31)) - 1u) : 0u;
+    while (m == 0 && w > 0) m = s_ends[--w];
+    return m ? w * 32 + 31 - __clz(m) : -1;
+  };
+  // a row's pieces in order: tails of groups [s, x), then the head of group x
+  auto chain = [&](int s, int x, bool head, float (&acc)[NV][V]) {
+    #pragma unroll
+    for (int j = 0; j < NV; j++) {
+      float comp[V];
+      const int c = lane * V + j * G * V;
+      #pragma unroll
+      for (int i = 0; i < V; i++) acc[j][i] = comp[i] = 0.f;
+      for (int k = max(s, 0); k < x; k++)
+        #pragma unroll
+        for (int i = 0; i < V; i++) kahan_add(acc[j][i], comp[i], s_tail[k * COLS + c + i]);
+      if (head)
+        #pragma unroll
+        for (int i = 0; i < V; i++) kahan_add(acc[j][i], comp[i], s_head[x * COLS + c + i]);
+    }
+  };
+  auto to_slot = [&](float *slots, float (&acc)[NV][V]) {
+    float *d = slots + (int64_t)tile * a.N + col0;
+    #pragma unroll
+    for (int j = 0; j < NV; j++)
+      if (act[j]) store_vec<float, V>(d + j * G * V, acc[j], strm);
+  };
+  float acc[NV][V];
+  if (hr) {
+    const int s = prev_end(g);
+    chain(s, g, true, acc);
+    if (s < 0 && has_head) {  // the row that entered the tile ends
+      to_slot(p.heads, acc);
+      tile_arrive<TC, G, V, NV, ADDC>(p, a.N, TILE, rlo - 1, lane, mask, phase, a.phases, col0, act, strm);
+    } else {
+      tile_store<TC, G, V, NV, ADDC>(p, a.N, hr - 1, acc, col0, act, strm);
+    }
+  }
+  if (g == 0 && te < p.nnz && __ldg(p.indptr + rhi) > te) {  // the last row goes on
+    const int s = prev_end(NG);
+    chain(s, NG, false, acc);
+    const bool whole = s < 0 && has_head;  // the tile lies inside one row
+    to_slot(whole ? p.heads : p.tails, acc);
+    tile_arrive<TC, G, V, NV, ADDC>(p, a.N, TILE, whole ? rlo - 1 : rhi - 1, lane, mask, phase, a.phases, col0, act,
+                                    strm);
+  }
+}
+
+template <typename T, typename TC>
+inline void *tile_ptr(int G, int V, int NV, bool addc) {
+#define SS_TILE(g, v, nv)           \
+  if (G == g && V == v && NV == nv) \
+    return addc ? (void *)eb_tile_kernel<T, TC, g, v, nv, true> : (void *)eb_tile_kernel<T, TC, g, v, nv, false>;
+#define SS_TILE_G(v) SS_TILE(1, v, 1) SS_TILE(2, v, 1) SS_TILE(4, v, 1) SS_TILE(8, v, 1) SS_TILE(16, v, 1)
+  SS_TILE_G(1) SS_TILE(16, 1, 2) SS_TILE(16, 1, 3) SS_TILE(16, 1, 4)
+  SS_TILE_G(2) SS_TILE(16, 2, 2)
+  SS_TILE_G(4)
+  if constexpr (sizeof(T) == 2) { SS_TILE_G(8) }
+#undef SS_TILE_G
+#undef SS_TILE
+  return nullptr;
+}
+
+// Kernel tables, one translation unit per pair of types.
+void *tile_kernel_f32(int G, int V, int NV, bool addc);
+void *tile_kernel_f32_bf16(int G, int V, int NV, bool addc);
+void *tile_kernel_f32_f16(int G, int V, int NV, bool addc);
+void *tile_kernel_bf16(int G, int V, int NV, bool addc);
+void *tile_kernel_bf16_f32(int G, int V, int NV, bool addc);
+void *tile_kernel_f16(int G, int V, int NV, bool addc);
+void *tile_kernel_f16_f32(int G, int V, int NV, bool addc);
+
+// Geometry of the walk over one matrix at width N.
+struct TileGeom {
+  int G, V, NV, phases;  // lanes, elements per vector, vectors per lane, column phases
+  int slog, tile;        // log2 of a piece, nonzeros of a tile
+  int tiles;
+  size_t smem;
+};
+// vmax: elements per vector that the alignment of B and C allows
+TileGeom tile_geom(int N, int nnz, int dtype, int vmax);
+// Launches the walk of `a` (a.items * a.phases blocks, `smem` bytes each).
+ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, cudaStream_t s);
+
+}  // namespace ss

@@ -103,6 +103,20 @@ int sm_count();
 // L2 size of the current device in bytes (cached per device).
 long long l2_bytes();
 
+// The tile walk (eb_tile.cu): ebsr with the chunk it chooses itself.
+bool tile_fits(int N, int nnz, int dtype);
+size_t tile_workspace_bytes(int N, int nnz, int dtype);
+int tile_vmax(const void *B, int b_bytes, const void *C, int c_bytes);
+ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s);
+// scratch of an ebsr call when it takes the group walk (abi.cu)
+size_t ebsr_walk_workspace(const ss_csr *A, int N, const ss_knobs *knobs);
+// ebsr tuples that ask for sequential runs of more than 2048 nonzeros
+// (thread_nz << group_factor) get the group walk with exactly those chunks
+// (less scratch, fewer partial sums); every other tuple gets the tile walk,
+// faster at every width and size measured (1e6 power-law: N = 64 FP32 203
+// against 242 us, N = 4 61 against 110 us, N = 128 BF16 258 against 341 us).
+inline bool tile_tuple(int group_factor, int thread_nz) { return ((long long)thread_nz << group_factor) <= 2048; }
+
 // Launchers (kernels live in spmm_rb.cu, eb_walk.cu, eb_scan.cu).
 ss_status launch_rbsr(const SpmmCall &c, const RbGeom &g, cudaStream_t s);
 ss_status launch_rbpr(const SpmmCall &c, const RbGeom &g, cudaStream_t s);

@@ -14,7 +14,8 @@
 //  * the array holds kNoallocScratchBytes (16 MiB) on every GPU that loads
 //    this library, for the life of the process;
 //  * a call whose scratch need (ss_spmm_workspace_size for SS_EBSR with the
-//    same A, N and knobs) is larger is rejected with SS_ERR_CAPACITY;
+//    same A, N and knobs, or the group walk's where that is smaller) is
+//    larger is rejected with SS_ERR_CAPACITY;
 //  * all calls on a device share the one array.  Calls that overlap on the
 //    GPU (different streams, or host threads that do not order them) race on
 //    it; serialise them.  Nothing in the array needs clearing by the
@@ -75,6 +76,10 @@ extern "C" ss_status ss_spmm_ebsr_noalloc(const ss_csr *A, int N, const void *B,
   size_t need = 0;
   ss_status st = ss_spmm_workspace_size(SS_EBSR, A, N, knobs, &need);
   if (st != SS_OK) return st;
+  if (need > kNoallocScratchBytes) {  // the group walk with the tuple's chunks may need less
+    const size_t walk = ebsr_walk_workspace(A, N, knobs);
+    if (walk < need) need = walk;
+  }
   if (need > kNoallocScratchBytes)
     return fail(SS_ERR_CAPACITY,
                 "ss_spmm_ebsr_noalloc: this call needs %zu bytes of scratch, above the fixed %zu bytes; "

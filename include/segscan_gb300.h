@@ -276,6 +276,14 @@ ss_status ss_coo_to_csr(int nrow, int nnz, const int32_t *rows,
                         const int32_t *cols, int32_t *indptr,
                         int32_t *out_cols, int32_t *perm, void *ws,
                         size_t ws_bytes, void *stream);
+/* The same with the edge values (SS_F32 / SS_BF16 / SS_F16, may be NULL with
+ * out_values) gathered into CSR order in the same pass. */
+ss_status ss_coo_to_csr_values(int nrow, int nnz, const int32_t *rows,
+                               const int32_t *cols, const void *values,
+                               int value_dtype, int32_t *indptr,
+                               int32_t *out_cols, int32_t *perm,
+                               void *out_values, void *ws, size_t ws_bytes,
+                               void *stream);
 
 /* out[p] = perm-gathered values: out[q] = values[perm[q]] (any dtype). */
 ss_status ss_gather_values(const void *values, int dtype, const int32_t *perm,

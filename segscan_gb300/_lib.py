@@ -81,6 +81,8 @@ _SIGNATURES = {
     "ss_device_error": (c_int, [POINTER(c_int), c_int]),
     "ss_selftest_bounded_wait": (c_int, [c_int, c_void_p]),
     "ss_coo_to_csr_workspace_size": (c_int, [c_int, c_int, POINTER(c_size_t)]),
+    "ss_coo_to_csr_values": (c_int, [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                     c_void_p, c_void_p, c_size_t, c_void_p]),
     "ss_coo_to_csr": (c_int, [c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
                               c_void_p]),
     "ss_mtx_read": (c_int, [c_char_p, c_int, POINTER(c_void_p)]),

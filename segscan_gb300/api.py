@@ -531,9 +531,15 @@ def coo_to_csr(nrow: int, rows: torch.Tensor, cols: torch.Tensor, ncol: Optional
     indptr = _output(nrow + 1, torch.int32, dev)
     out_cols = _output(nnz, torch.int32, dev)
     perm = _output(nnz, torch.int32, dev)
-    _lib.call("ss_coo_to_csr", nrow, nnz, _ptr(rows), _ptr(cols), _ptr(indptr), _ptr(out_cols), _ptr(perm), wp, wn,
-              _stream(stream))
-    vals = gather_values(values, perm, stream) if values is not None else None
+    vals, code = None, Dtype.F32
+    if values is not None:  # gathered along with the columns
+        if values.numel() != nnz:
+            raise ValueError(f"perm ({nnz}) and values ({values.numel()}) differ in length")
+        _need_cuda("values", values)
+        code = dtype_code(values.dtype)
+        vals = _output(values.shape, values.dtype, values.device)
+    _lib.call("ss_coo_to_csr_values", nrow, nnz, _ptr(rows), _ptr(cols), _ptr(values), int(code), _ptr(indptr),
+              _ptr(out_cols), _ptr(perm), _ptr(vals), wp, wn, _stream(stream))
     K = int(ncol) if ncol is not None else (int(cols.max()) + 1 if nnz else 0)
     return CsrMatrix(nrow, K, indptr, out_cols, vals), perm
 

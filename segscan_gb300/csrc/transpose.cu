@@ -28,8 +28,9 @@
 // Order inside a column before step 4's sort depends on atomics; after it,
 // only on the input, so repeated calls agree.
 //
-// ss_coo_to_csr (and ss_csr_transpose beyond TB_NB_MAX buckets of 8192
-// columns): a one-level counting sort,
+// ss_coo_to_csr takes the stable sort of stable_sort.cu up to 16.7 M rows.
+// Beyond, for a workspace that only it fits, and for ss_csr_transpose beyond
+// TB_NB_MAX buckets of 8192 columns: a one-level counting sort,
 //   1. key histogram (atomics)               -> counts
 //   2. exclusive scan of counts (3 kernels; 5 when K > 4096^2, the tile
 //      sums then scanned in two levels)      -> t_indptr
@@ -43,6 +44,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "stable_sort.cuh"
 
 namespace ss {
 
@@ -706,7 +708,7 @@ __device__ void sort_segment(int32_t *seg, int n, int32_t *stage, int cap) {
   __syncthreads();
 }
 
-struct SortArgs {
+struct BucketSortArgs {
   const int32_t *start, *pos, *row, *col;
   int K, NB, f, F, cap;
   int32_t *t_indptr, *perm, *t_indices;
@@ -735,7 +737,7 @@ __device__ __forceinline__ void sort_short_columns(int32_t *kp, int32_t *vp, con
 
 // t_vals[s0 + i] = vals[src[i]] for the bucket's n entries, eight gathers
 // in flight per thread; src is shared or global, the call site fixes which.
-__device__ __forceinline__ void gather_bucket_values(const SortArgs &a, const int32_t *src, int s0, int n) {
+__device__ __forceinline__ void gather_bucket_values(const BucketSortArgs &a, const int32_t *src, int s0, int n) {
   for (int i0 = 0; i0 < n; i0 += 8 * blockDim.x) {
     uint32_t v[8];
     #pragma unroll
@@ -758,7 +760,7 @@ __device__ __forceinline__ void gather_bucket_values(const SortArgs &a, const in
 // from the 16-byte word holding its first record to the one holding its
 // last, completing on bar.  Returns the offset of the first record in the
 // staged arrays (0..3).  Thread 0 only.
-__device__ __forceinline__ int stage_bucket(const SortArgs &a, int b, int32_t *rc, int32_t *rp, int32_t *rr,
+__device__ __forceinline__ int stage_bucket(const BucketSortArgs &a, int b, int32_t *rc, int32_t *rp, int32_t *rr,
                                             uint64_t *bar) {
   const int s0 = __ldg(a.start + b), n = __ldg(a.start + b + 1) - s0;
   const int w0 = s0 & ~3, w1 = (s0 + n + 3) & ~3;
@@ -777,7 +779,7 @@ __device__ __forceinline__ int stage_bucket(const SortArgs &a, int b, int32_t *r
 // columns are counted, its records placed by column and sorted inside each
 // column, all in shared memory.  A larger bucket is placed and sorted in
 // the output arrays.
-__global__ void __launch_bounds__(TB_ST, TB_SORT_BLOCKS) bucket_sort_kernel(SortArgs a) {
+__global__ void __launch_bounds__(TB_ST, TB_SORT_BLOCKS) bucket_sort_kernel(BucketSortArgs a) {
   extern __shared__ __align__(16) int32_t sm[];
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm);  // [4 ints]
   const int stg = a.cap + 8;          // staged array length (alignment slack; a multiple of 4)
@@ -951,7 +953,7 @@ static ss_status bucket_transpose(const ss_csr *A, const BucketPlan &pl, int32_t
   pa.M = M; pa.K = K; pa.nnz = nnz; pa.f = pl.f; pa.NB = pl.NB;
   pa.cursor = w.cursor; pa.pos = w.pos; pa.row = w.row; pa.col = w.col;
   bucket_partition_kernel<<<(int)std::min<long long>(tiles, (long long)sms * TB_PART_BLOCKS), TB_PT, part_smem, s>>>(pa);
-  SortArgs sa;
+  BucketSortArgs sa;
   sa.start = w.start; sa.pos = w.pos; sa.row = w.row; sa.col = w.col;
   sa.K = K; sa.NB = pl.NB; sa.f = pl.f; sa.F = pl.F; sa.cap = pl.cap;
   sa.t_indptr = t_indptr; sa.perm = perm; sa.t_indices = t_indices;
@@ -1021,26 +1023,46 @@ ss_status ss_csr_transpose(const ss_csr *A, int32_t *t_indptr, int32_t *t_indice
 
 ss_status ss_coo_to_csr_workspace_size(int nrow, int nnz, size_t *bytes) {
   if (!bytes || nrow < 0 || nnz < 0) return fail(SS_ERR_INVALID_ARG, "bad arguments");
-  *bytes = transpose_ws_bytes(nrow, nnz, nullptr, nullptr);
+  const StableSortPlan sp = stable_sort_plan(nrow, nnz);
+  *bytes = sp.ok ? stable_sort_ws(sp, nnz) : transpose_ws_bytes(nrow, nnz, nullptr, nullptr);
   return SS_OK;
 }
 
-ss_status ss_coo_to_csr(int nrow, int nnz, const int32_t *rows, const int32_t *cols, int32_t *indptr,
-                        int32_t *out_cols, int32_t *perm, void *ws, size_t ws_bytes, void *stream) {
+ss_status ss_coo_to_csr_values(int nrow, int nnz, const int32_t *rows, const int32_t *cols, const void *values,
+                               int value_dtype, int32_t *indptr, int32_t *out_cols, int32_t *perm, void *out_values,
+                               void *ws, size_t ws_bytes, void *stream) {
   ss::NvtxRange nvtx_range("ss_coo_to_csr");
   if (nrow < 0 || nnz < 0 || !indptr || (nnz > 0 && (!rows || !cols || !out_cols || !perm)))
     return fail(SS_ERR_INVALID_ARG, "bad arguments");
-  const size_t need = transpose_ws_bytes(nrow, nnz, nullptr, nullptr);
+  if (out_values && ((nnz > 0 && !values) || value_dtype < SS_F32 || value_dtype > SS_F16))
+    return fail(SS_ERR_INVALID_ARG, "out_values given without values of a known dtype");
+  const StableSortPlan sp = stable_sort_plan(nrow, nnz);
+  const bool stable = sp.ok && ws_bytes >= stable_sort_ws(sp, nnz);
+  const size_t need = stable ? stable_sort_ws(sp, nnz) : transpose_ws_bytes(nrow, nnz, nullptr, nullptr);
   if (ws_bytes < need || !ws || ((uintptr_t)ws % 256))
     return fail(SS_ERR_WORKSPACE, "workspace needs %zu bytes (256-byte aligned), got %zu", need, ws_bytes);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (stable) {
+    SortArgs a{};
+    a.keys = rows; a.payload = cols; a.vals = out_values ? values : nullptr;
+    a.K = nrow; a.nnz = nnz; a.vsize = dtype_size(value_dtype);
+    a.out_indptr = indptr; a.perm = perm; a.out_payload = out_cols; a.out_vals = out_values;
+    return stable_sort(sp, a, ws, s);
+  }
   TransposeWs w;
   transpose_ws_bytes(nrow, nnz, &w, ws);
-  cudaStream_t s = (cudaStream_t)stream;
   ss_status st = counting_sort(rows, nnz, nrow, indptr, perm, w, s);
   if (st != SS_OK || nnz == 0 || nrow == 0) return st;
   gather_rows_kernel<<<grid_for(nnz, 256), 256, 0, s>>>(perm, cols, nnz, out_cols);
   cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? SS_OK : cuda_fail(e, "coo to csr launch");
+  if (e != cudaSuccess) return cuda_fail(e, "coo to csr launch");
+  return out_values ? ss_gather_values(values, value_dtype, perm, nnz, out_values, stream) : SS_OK;
+}
+
+ss_status ss_coo_to_csr(int nrow, int nnz, const int32_t *rows, const int32_t *cols, int32_t *indptr,
+                        int32_t *out_cols, int32_t *perm, void *ws, size_t ws_bytes, void *stream) {
+  return ss_coo_to_csr_values(nrow, nnz, rows, cols, nullptr, SS_F32, indptr, out_cols, perm, nullptr, ws, ws_bytes,
+                              stream);
 }
 
 }  // extern "C"

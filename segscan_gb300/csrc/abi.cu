@@ -494,6 +494,11 @@ static ss_status seg_geometry(int seg_strategy, int nnz, int N, int dtype, const
   return fail(SS_ERR_INVALID_ARG, "unknown segment strategy %d", seg_strategy);
 }
 
+static bool seg_takes_tile(int seg_strategy, const ss_knobs &k, int N, int nnz) {
+  return seg_strategy == SS_SEG_SR && nnz > 0 && N > 0 && tile_tuple(k.group_factor, k.thread_nz) &&
+         seg_tile_fits(N, nnz);
+}
+
 static void seg_default_knobs(int seg_strategy, ss_knobs &k) {
   memset(&k, 0, sizeof(k));
   k.thread_per_block = 256;
@@ -523,6 +528,7 @@ ss_status ss_segment_coo_workspace_size(int seg_strategy, int nnz, int N, const 
     const size_t need = seg_strategy == SS_SEG_SR ? seg_sr_workspace_bytes(g, N) : eb_workspace_bytes(g, N);
     if (need > most) most = need;
   }
+  if (seg_takes_tile(seg_strategy, *knobs, N, nnz)) most = seg_tile_workspace_bytes(N, nnz);
   *bytes = most;
   return SS_OK;
 }
@@ -552,7 +558,14 @@ ss_status ss_segment_coo(int seg_strategy, const void *src, int src_dtype, const
     cudaError_t e = cudaMemsetAsync(dst, 0, (size_t)dst_len * N * sizeof(float), s);
     return e == cudaSuccess ? SS_OK : cuda_fail(e, "zero dst");
   }
-  const size_t need = seg_strategy == SS_SEG_SR ? seg_sr_workspace_bytes(g, N) : eb_workspace_bytes(g, N);
+  size_t need = seg_strategy == SS_SEG_SR ? seg_sr_workspace_bytes(g, N) : eb_workspace_bytes(g, N);
+  bool tile = false;
+  if (seg_takes_tile(seg_strategy, *knobs, N, nnz)) {
+    // a workspace that only the group walk fits still gets that walk
+    const size_t tneed = seg_tile_workspace_bytes(N, nnz);
+    tile = ws_bytes >= tneed;
+    if (tile || tneed < need) need = tneed;
+  }
   if (ws_bytes < need || !ws || ((uintptr_t)ws % 256))
     return fail(SS_ERR_WORKSPACE, "workspace needs %zu bytes (256-byte aligned), got %zu", need, ws_bytes);
   SegCall c;
@@ -564,6 +577,7 @@ ss_status ss_segment_coo(int seg_strategy, const void *src, int src_dtype, const
     c.accumulate = 1;
   }
   c.kahan_threshold = knobs->kahan_threshold > 0 ? knobs->kahan_threshold : 1024;
+  if (tile) return launch_seg_tile(c, g.chunk > c.kahan_threshold, ws, s);
   return seg_strategy == SS_SEG_SR ? launch_seg_sr(c, g, ws, s) : launch_seg_pr(c, g, ws, s);
 }
 

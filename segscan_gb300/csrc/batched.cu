@@ -80,7 +80,7 @@ static ss_status batch_layout(int count, const ss_csr *mats, int N, const ss_kno
       memset(&p, 0, sizeof(p));
       p.indptr = A.indptr; p.cols = A.indices; p.vals = A.values;
       p.M = A.nrow; p.K = A.ncol; p.nnz = A.nnz;
-      p.slog = g.slog;
+      p.piece = g.piece; p.inv_piece = inverse_of(g.piece);
       p.item_begin = (int)titems;
       p.wide = (((uintptr_t)A.indices | (uintptr_t)A.values) & 15u) == 0;
       p.index = m;

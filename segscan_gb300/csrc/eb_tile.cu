@@ -2,7 +2,7 @@
 #include <algorithm>
 #include <cstring>
 
-#include "eb_tile.cuh"
+#include "seg_tile.cuh"
 
 namespace ss {
 
@@ -11,15 +11,15 @@ namespace ss {
 // counts, so the walk needs no memset of its own.  2 us on a million rows,
 // against 2.5 us of search latency in every block of the walk (N = 64:
 // 207 -> 203 us).
-__global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restrict__ indptr, int M, int log2_tile,
+__global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restrict__ indptr, int M, int tile,
                                                         int tiles, int32_t *__restrict__ row_start,
                                                         int *__restrict__ cnt, int ncnt) {
   const long long stride = (long long)gridDim.x * 256, i0 = blockIdx.x * 256ll + threadIdx.x;
   for (long long r0 = i0 * 4; r0 <= M; r0 += stride * 4) {
     int x[5];
-    x[0] = r0 > 0 ? __ldg(indptr + r0 - 1) >> log2_tile : -1;
+    x[0] = r0 > 0 ? __ldg(indptr + r0 - 1) / tile : -1;
     #pragma unroll
-    for (int i = 0; i < 4; i++) x[i + 1] = r0 + i <= M ? __ldg(indptr + r0 + i) >> log2_tile : INT_MIN;
+    for (int i = 0; i < 4; i++) x[i + 1] = r0 + i <= M ? __ldg(indptr + r0 + i) / tile : INT_MIN;
     #pragma unroll
     for (int i = 0; i < 4; i++)
       for (int t = max(x[i] + 1, 0); t <= min(x[i + 1], tiles - 1); t++) row_start[t] = (int)r0 + i;
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restric
   for (long long i = i0; i < ncnt; i += stride) cnt[i] = 0;
 }
 
-TileGeom tile_geom(int N, int nnz, int dtype, int vmax) {
+TileGeom tile_geom(int N, int nnz, int dtype, int vmax, bool seg) {
   TileGeom g;
   int V = std::min(16 / dtype_size(dtype), std::max(1, vmax));
   while (N % V) V >>= 1;
@@ -36,6 +36,11 @@ TileGeom tile_geom(int N, int nnz, int dtype, int vmax) {
   g.V = V;
   g.NV = 1;
   g.G = std::min(16, ceil_pow2(nv));
+  // 17 to 32 wide vectors: one phase of 32 lanes instead of two of 16, unless
+  // two full phases gather a matrix's rows as fast (N = 128: 420 against 428
+  // us).  A half empty second phase costs more (N = 100 BF16: ## -> ## us),
+  // and streamed rows are better read in one piece.
+  if (V >= 4 && nv > 16 && nv <= 32 && (seg || nv < 32)) g.G = 32;
   // widths that no wide vector divides: several vectors per lane, as many as
   // leave the fewest idle columns (N = 47: 16 lanes of three, 108 us, against
   // three phases of one, 252 us)
@@ -44,16 +49,24 @@ TileGeom tile_geom(int N, int nnz, int dtype, int vmax) {
     for (int m = 2; m <= most; m++)
       if (ceil_div(nv, 16 * m) * m <= ceil_div(nv, 16 * g.NV) * g.NV) g.NV = m;
   g.phases = ceil_div(N, g.G * V * g.NV);
-  // pieces as long as shared memory allows without costing resident blocks
-  // (2048 nonzeros a tile, 1024 with 16 lanes), shorter where a matrix would
-  // otherwise fill less than two blocks per SM
+  // Pieces as long as shared memory allows without costing resident blocks
+  // (2048 nonzeros a tile, 1024 with 16 or 32 lanes): a block's set-up is
+  // about a quarter of its time there.  Shorter where two blocks per SM would
+  // not be filled (more, shorter blocks than that are slower: 320 K nonzeros
+  // BF16 N = 64 18 us at 313 blocks, 20 at 625, 25 at 1250), and cut so that
+  // a few waves of blocks are whole ones.
   const int NG = TW_T / g.G;
-  int slog = g.G >= 16 ? 6 : 3 + ilog2(g.G);
-  while (slog > 3 && (long long)nnz < ((long long)NG << slog) * 2 * sm_count()) slog--;
-  g.slog = slog;
-  g.tile = NG << slog;
+  const int most_piece = g.G >= 32 ? 128 : g.G >= 16 ? 64 : 8 * g.G;
+  const long long work = (long long)nnz * g.phases;             // nonzeros over the column phases
+  const long long wave = 4LL * sm_count() * NG, half = wave / 2;  // groups of a resident wave
+  long long piece = most_piece;
+  if (work <= half * most_piece) piece = ceil_div(work, half);
+  else if (work > wave * most_piece && work <= 6 * wave * most_piece)
+    piece = ceil_div(work, wave * ceil_div(work, wave * most_piece));
+  g.piece = (int)std::max(8LL, (piece + 3) / 4 * 4);
+  g.tile = NG * g.piece;
   g.tiles = std::max(1, ceil_div(nnz, g.tile));
-  g.smem = (size_t)tile_smem(g.G, V * g.NV, slog).total * 4;
+  g.smem = (size_t)tile_smem(g.G, V * g.NV, g.piece).total * 4;
   return g;
 }
 
@@ -119,7 +132,7 @@ ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
   TileProb &p = a.p;
   p.indptr = c.indptr; p.cols = c.indices; p.vals = c.vals; p.B = c.B; p.C = c.C;
   p.M = c.M; p.K = c.K; p.nnz = c.nnz;
-  p.slog = g.slog;
+  p.piece = g.piece; p.inv_piece = inverse_of(g.piece);
   p.wide = (((uintptr_t)c.indices | (uintptr_t)c.vals) & 15u) == 0;
   char *w = (char *)ws;
   p.cnt = (int *)w; w += align256((size_t)g.tiles * g.phases * 4);
@@ -132,11 +145,64 @@ ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
   a.keep_frac = l2_keep_fraction((size_t)c.K * c.N * dtype_size(c.val_dtype));
   const int ncnt = g.tiles * g.phases;
   const long long want = ((long long)c.M + 1024) / 1024;
-  tile_rows_kernel<<<(unsigned)std::min(want, (long long)sm_count() * 16), 256, 0, s>>>(c.indptr, c.M, ilog2(g.tile), g.tiles,
+  tile_rows_kernel<<<(unsigned)std::min(want, (long long)sm_count() * 16), 256, 0, s>>>(c.indptr, c.M, g.tile, g.tiles,
                                                                                       row_start, p.cnt, ncnt);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "tile rows launch");
   return run_tile(c.val_dtype, c.c_dtype, g, g.smem, a, s);
+}
+
+// ---------------------------------------------------------------------
+// segment_coo
+// ---------------------------------------------------------------------
+static size_t seg_tile_ws(const TileGeom &g, int N) {
+  return align256((size_t)g.tiles * g.phases * 4) + align256((size_t)2 * g.tiles * 4) +
+         2 * (size_t)g.tiles * (size_t)N * sizeof(float);
+}
+
+bool seg_tile_fits(int N, int nnz) {
+  if (N >= (1 << 29)) return false;
+  for (int dt : {SS_F32, SS_BF16})
+    for (int v = 1; v <= 16 / dtype_size(dt); v <<= 1) {
+      const TileGeom g = tile_geom(N, nnz, dt, v, true);
+      if (g.tiles > 1 << 18 || (long long)g.tiles * g.phases >= (1LL << 31)) return false;
+    }
+  return true;
+}
+
+size_t seg_tile_workspace_bytes(int N, int nnz) {
+  size_t most = 0;  // over the source types and the alignments of src and dst
+  for (int dt : {SS_F32, SS_BF16})
+    for (int v = 1; v <= 16 / dtype_size(dt); v <<= 1)
+      most = std::max(most, seg_tile_ws(tile_geom(N, nnz, dt, v, true), N));
+  return most;
+}
+
+ss_status launch_seg_tile(const SegCall &c, bool kahan, void *ws, cudaStream_t s) {
+  const TileGeom g = tile_geom(c.N, c.nnz, c.src_dtype, tile_vmax(c.src, dtype_size(c.src_dtype), c.dst, 4), true);
+  SegTileArgs a;
+  memset(&a, 0, sizeof(a));
+  a.src = c.src; a.index = c.index; a.dst = c.dst;
+  a.M = c.dst_len; a.nnz = c.nnz; a.N = c.N; a.piece = g.piece; a.inv_piece = inverse_of(g.piece); a.tiles = g.tiles; a.phases = g.phases;
+  a.reduce = c.reduce; a.kahan = kahan;
+  char *w = (char *)ws;
+  const size_t cnt_bytes = align256((size_t)g.tiles * g.phases * 4);
+  a.cnt = (int *)w; w += cnt_bytes;
+  a.hcnt = (int *)w;
+  a.tcnt = a.hcnt + g.tiles; w += align256((size_t)2 * g.tiles * 4);
+  a.heads = (float *)w;
+  a.tails = a.heads + (size_t)g.tiles * c.N;
+  void *fn = c.src_dtype == SS_F32    ? seg_tile_kernel_f32(g.G, g.V, g.NV, c.accumulate != 0)
+             : c.src_dtype == SS_BF16 ? seg_tile_kernel_bf16(g.G, g.V, g.NV, c.accumulate != 0)
+                                      : seg_tile_kernel_f16(g.G, g.V, g.NV, c.accumulate != 0);
+  if (!fn) return fail(SS_ERR_UNSUPPORTED_KNOBS, "no segment tile walk for G=%d V=%d NV=%d", g.G, g.V, g.NV);
+  cudaError_t e = cudaMemsetAsync(a.cnt, 0, (size_t)g.tiles * g.phases * 4, s);
+  if (e != cudaSuccess) return cuda_fail(e, "segment arrival counts");
+  const int NG = TW_T / g.G;
+  const size_t smem = ((size_t)NG * (g.piece + 4) + 2 * (size_t)TW_T * g.V * g.NV + ceil_div(g.tile, 32)) * 4;
+  void *args[] = {&a};
+  e = cudaLaunchKernel(fn, dim3((unsigned)(g.tiles * g.phases), 1, 1), dim3(TW_T, 1, 1), args, smem, s);
+  return e == cudaSuccess ? SS_OK : cuda_fail(e, "segment tile walk launch");
 }
 
 }  // namespace ss

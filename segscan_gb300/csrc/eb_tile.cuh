@@ -48,11 +48,11 @@ struct __align__(16) TileProb {
   int *cnt;                  // [tiles * phases] arrivals per straddling row
   float *heads, *tails;      // [tiles * N] partials of a tile's first / last row
   int M, K, nnz;
-  int slog;        // a piece is 1 << slog nonzeros
+  int piece;       // nonzeros per group, a multiple of four
+  uint32_t inv_piece;
   int item_begin;  // first block of this matrix (batched)
   int wide;        // columns and values may be loaded 16 bytes at a time
   int index;       // host: the matrix's place in its batch
-  int pad;
 };
 
 struct TileArgs {
@@ -68,8 +68,8 @@ struct TileArgs {
 struct TileSmem {
   int col, val, info, head, tail, kb, ends, total;
 };
-__host__ __device__ inline TileSmem tile_smem(int G, int E, int slog) {
-  const int NG = TW_T / G, words = NG * ((1 << slog) + 4);
+__host__ __device__ inline TileSmem tile_smem(int G, int E, int piece) {
+  const int NG = TW_T / G, words = NG * (piece + 4);
   TileSmem s;
   int o = (int)sizeof(TileProb) / 4;
   s.col = o; o += words;
@@ -77,11 +77,15 @@ __host__ __device__ inline TileSmem tile_smem(int G, int E, int slog) {
   s.info = o; o += words;
   s.head = o; o += TW_T * E;
   s.tail = o; o += TW_T * E;
-  s.kb = o; o += ((NG << slog) + 31) / 32;
+  s.kb = o; o += (NG * piece + 31) / 32;
   s.ends = o; o += (NG + 31) / 32;
   s.total = o;
   return s;
 }
+
+// e / piece for e below 2^16 and inv = ceil(2^32 / piece)
+__device__ __forceinline__ int piece_of(int e, uint32_t inv) { return (int)__umulhi((uint32_t)e, inv); }
+inline uint32_t inverse_of(int piece) { return (uint32_t)(((1ull << 32) + piece - 1) / piece); }
 
 template <int V>
 __device__ __forceinline__ void store_smem(float *p, const float (&v)[V]) {
@@ -123,46 +127,46 @@ __device__ __forceinline__ void load_old(const TC *p, float (&out)[V]) {
   }
 }
 
-// One predicated instruction each, so that groups of one warp do not branch
-// apart where only some of them end a row.
-__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[4], uint64_t pol, bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %6, 0;\n"
+// One predicated instruction each (where on > 0), so that groups of one warp
+// do not branch apart where only some of them end a row.
+__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[4], uint64_t pol, int on) {
+  asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %6, 0;\n"
                " @p st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %5;\n}" ::"l"(p), "r"(w[0]), "r"(w[1]),
-               "r"(w[2]), "r"(w[3]), "l"(pol), "r"((unsigned)on) : "memory");
+               "r"(w[2]), "r"(w[3]), "l"(pol), "r"(on) : "memory");
 }
-__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[2], uint64_t pol, bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[2], uint64_t pol, int on) {
+  asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %4, 0;\n"
                " @p st.global.L2::cache_hint.v2.u32 [%0], {%1, %2}, %3;\n}" ::"l"(p), "r"(w[0]), "r"(w[1]), "l"(pol),
-               "r"((unsigned)on) : "memory");
+               "r"(on) : "memory");
 }
-__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[1], uint64_t pol, bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.global.L2::cache_hint.u32 [%0], %1, %2;\n}" ::
-               "l"(p), "r"(w[0]), "l"(pol), "r"((unsigned)on) : "memory");
+__device__ __forceinline__ void st_if(void *p, const uint32_t (&w)[1], uint64_t pol, int on) {
+  asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %3, 0;\n @p st.global.L2::cache_hint.u32 [%0], %1, %2;\n}" ::
+               "l"(p), "r"(w[0]), "l"(pol), "r"(on) : "memory");
 }
-__device__ __forceinline__ void st16_if(void *p, uint16_t w, uint64_t pol, bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.global.L2::cache_hint.u16 [%0], %1, %2;\n}" ::
-               "l"(p), "h"(w), "l"(pol), "r"((unsigned)on) : "memory");
+__device__ __forceinline__ void st16_if(void *p, uint16_t w, uint64_t pol, int on) {
+  asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %3, 0;\n @p st.global.L2::cache_hint.u16 [%0], %1, %2;\n}" ::
+               "l"(p), "h"(w), "l"(pol), "r"(on) : "memory");
 }
-__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[4], bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n @p ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n}"
-               : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]) : "l"(p), "r"((unsigned)on) : "memory");
+__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[4], int on) {
+  asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %5, 0;\n @p ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n}"
+               : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]) : "l"(p), "r"(on) : "memory");
 }
-__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[2], bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p ld.global.v2.u32 {%0, %1}, [%2];\n}"
-               : "+r"(w[0]), "+r"(w[1]) : "l"(p), "r"((unsigned)on) : "memory");
+__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[2], int on) {
+  asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %3, 0;\n @p ld.global.v2.u32 {%0, %1}, [%2];\n}"
+               : "+r"(w[0]), "+r"(w[1]) : "l"(p), "r"(on) : "memory");
 }
-__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[1], bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.global.u32 %0, [%1];\n}"
-               : "+r"(w[0]) : "l"(p), "r"((unsigned)on) : "memory");
+__device__ __forceinline__ void ld_if(const void *p, uint32_t (&w)[1], int on) {
+  asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %2, 0;\n @p ld.global.u32 %0, [%1];\n}"
+               : "+r"(w[0]) : "l"(p), "r"(on) : "memory");
 }
-__device__ __forceinline__ void ld16_if(const void *p, uint32_t &w, bool on) {
+__device__ __forceinline__ void ld16_if(const void *p, uint32_t &w, int on) {
   uint16_t h = 0;
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.global.u16 %0, [%1];\n}"
-               : "+h"(h) : "l"(p), "r"((unsigned)on) : "memory");
+  asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %2, 0;\n @p ld.global.u16 %0, [%1];\n}"
+               : "+h"(h) : "l"(p), "r"(on) : "memory");
   w = h;
 }
 template <typename T, int V>
-__device__ __forceinline__ void store_vec_if(T *p, const float (&v)[V], uint64_t pol, bool on) {
+__device__ __forceinline__ void store_vec_if(T *p, const float (&v)[V], uint64_t pol, int on) {
   if constexpr (V * sizeof(T) > 16) {
     constexpr int H = V / 2;
     float lo[H], hi[H];
@@ -190,7 +194,7 @@ struct OldVec {
   uint32_t w[P][W];
 };
 template <typename T, int V>
-__device__ __forceinline__ void load_old_if(const T *p, OldVec<T, V> &o, bool on) {
+__device__ __forceinline__ void load_old_if(const T *p, OldVec<T, V> &o, int on) {
   #pragma unroll
   for (int k = 0; k < OldVec<T, V>::P; k++) {
     const char *q = (const char *)p + 16 * k;
@@ -328,11 +332,10 @@ __device__ __forceinline__ int tile_walk(const TileProb &p, int N, int S, const 
         for (int i = 0; i < V; i++) acc[j][i] = fmaf(v, b[i], acc[j][i]);
       }
     }
-    const bool first = end != 0 && hr == 0;
-    const bool out = end != 0 && hr != 0;
+    const int out = hr ? end : 0;  // a row end after the first: stored here
     #pragma unroll
     for (int j = 0; j < NV; j++) {
-      if (first) store_smem<V>(shead + j * G * V, acc[j]);
+      if (end != out) store_smem<V>(shead + j * G * V, acc[j]);
       TC *d = (TC *)(Cj[j] + (uint64_t)(uint32_t)end * ldc);
       if (ADDC) {
         float x[V];
@@ -349,7 +352,7 @@ __device__ __forceinline__ int tile_walk(const TileProb &p, int N, int S, const 
         if (SLOW) comp[j][i] = end ? 0.f : comp[j][i];
       }
     }
-    hr = first ? end : hr;
+    hr = hr ? hr : end;
   };
   #pragma unroll 1
   for (int q = 0; q < S; q += 4) {
@@ -363,7 +366,7 @@ __device__ __forceinline__ int tile_walk(const TileProb &p, int N, int S, const 
       for (int u = 0; u < 4; u++)
         #pragma unroll
         for (int j = 0; j < NV; j++)
-          load_old_if<TC, V>((const TC *)(Cj[j] + (uint64_t)(uint32_t)is[u] * ldc), old[u][j], is[u] != 0);
+          load_old_if<TC, V>((const TC *)(Cj[j] + (uint64_t)(uint32_t)is[u] * ldc), old[u][j], is[u]);
     }
     const uint32_t k4 = SLOW ? kb[(p0 + q) >> 5] >> ((p0 + q) & 31) : 0u;
     consume(0, v4.x, i4.x, k4 & 1u);
@@ -400,8 +403,8 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
   }
   __syncthreads();
   const TileProb &p = *reinterpret_cast<const TileProb *>(smem);
-  const int S = 1 << p.slog, TILE = NG << p.slog;
-  const TileSmem L = tile_smem(G, E, p.slog);
+  const int S = p.piece, TILE = NG * S;
+  const TileSmem L = tile_smem(G, E, S);
   int32_t *s_col = smem + L.col, *s_info = smem + L.info;
   float *s_val = (float *)(smem + L.val), *s_head = (float *)(smem + L.head), *s_tail = (float *)(smem + L.tail);
   uint32_t *s_kb = (uint32_t *)(smem + L.kb), *s_ends = (uint32_t *)(smem + L.ends);
@@ -449,7 +452,7 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
         c[i] = -1;
         slow = true;
       }
-    const int w = e + 4 * (e >> p.slog);
+    const int w = e + 4 * piece_of(e, p.inv_piece);
     *reinterpret_cast<int4 *>(s_col + w) = make_int4(c[0], c[1], c[2], c[3]);
     *reinterpret_cast<float4 *>(s_val + w) = make_float4(v[0], v[1], v[2], v[3]);
     *reinterpret_cast<int4 *>(s_info + w) = make_int4(0, 0, 0, 0);
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
       }
       empty = s == e;
       const unsigned pos = (unsigned)(e - 1 - ts);
-      if (!empty && pos < (unsigned)n) s_info[pos + 4 * (pos >> p.slog)] = r + 1;
+      if (!empty && pos < (unsigned)n) s_info[pos + 4 * piece_of(pos, p.inv_piece)] = r + 1;
       if (e - s > a.kahan) {
         const int k0 = max(s - ts, 0), k1 = min(e - ts, n) - 1;
         for (int w = k0 >> 5; w <= k1 >> 5; w++) {
@@ -510,7 +513,7 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
   }
   slow = __syncthreads_or(slow);
   {
-    const int WN = (32 / G) << p.slog, w0 = (tid >> 5) * WN;  // the warp's nonzeros
+    const int WN = (32 / G) * S, w0 = (tid >> 5) * WN;  // the warp's nonzeros
     for (int w = w0 >> 5; w <= (w0 + WN - 1) >> 5; w++) slow |= s_kb[w] != 0;
   }
   const int gb = g * (S + 4);
@@ -582,8 +585,8 @@ inline void *tile_ptr(int G, int V, int NV, bool addc) {
 #define SS_TILE_G(v) SS_TILE(1, v, 1) SS_TILE(2, v, 1) SS_TILE(4, v, 1) SS_TILE(8, v, 1) SS_TILE(16, v, 1)
   SS_TILE_G(1) SS_TILE(16, 1, 2) SS_TILE(16, 1, 3) SS_TILE(16, 1, 4)
   SS_TILE_G(2) SS_TILE(16, 2, 2)
-  SS_TILE_G(4)
-  if constexpr (sizeof(T) == 2) { SS_TILE_G(8) }
+  SS_TILE_G(4) SS_TILE(32, 4, 1)
+  if constexpr (sizeof(T) == 2) { SS_TILE_G(8) SS_TILE(32, 8, 1) }
 #undef SS_TILE_G
 #undef SS_TILE
   return nullptr;
@@ -601,12 +604,13 @@ void *tile_kernel_f16_f32(int G, int V, int NV, bool addc);
 // Geometry of the walk over one matrix at width N.
 struct TileGeom {
   int G, V, NV, phases;  // lanes, elements per vector, vectors per lane, column phases
-  int slog, tile;        // log2 of a piece, nonzeros of a tile
+  int piece, tile;       // nonzeros of a piece and of a tile
   int tiles;
   size_t smem;
 };
-// vmax: elements per vector that the alignment of B and C allows
-TileGeom tile_geom(int N, int nnz, int dtype, int vmax);
+// vmax: elements per vector that the alignment of B and C allows; seg: the
+// segment walk, whose rows stream instead of being gathered
+TileGeom tile_geom(int N, int nnz, int dtype, int vmax, bool seg = false);
 // Launches the walk of `a` (a.items * a.phases blocks, `smem` bytes each).
 ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, cudaStream_t s);
 

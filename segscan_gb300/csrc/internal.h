@@ -108,6 +108,10 @@ bool tile_fits(int N, int nnz, int dtype);
 size_t tile_workspace_bytes(int N, int nnz, int dtype);
 int tile_vmax(const void *B, int b_bytes, const void *C, int c_bytes);
 ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s);
+// the segment form of it; kahan: every element summed with compensation
+bool seg_tile_fits(int N, int nnz);
+size_t seg_tile_workspace_bytes(int N, int nnz);
+ss_status launch_seg_tile(const SegCall &c, bool kahan, void *ws, cudaStream_t s);
 // scratch of an ebsr call when it takes the group walk (abi.cu)
 size_t ebsr_walk_workspace(const ss_csr *A, int N, const ss_knobs *knobs);
 // ebsr tuples that ask for sequential runs of more than 2048 nonzeros

@@ -1,0 +1,6 @@
+// FP16 instantiations of the segment tile walk.
+#include "seg_tile.cuh"
+
+namespace ss {
+void *seg_tile_kernel_f16(int G, int V, int NV, bool addc) { return seg_tile_ptr<__half>(G, V, NV, addc); }
+}  // namespace ss

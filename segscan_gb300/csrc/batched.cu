@@ -253,7 +253,7 @@ ss_status ss_spmm_batched(const void *host_plan, void *dev_plan, void *stream) {
     g.G = h.tG;
     g.V = h.tV;
     g.NV = h.tNV;
-    ss_status st = run_tile(h.val_dtype, h.c_dtype, g, h.tsmem, a, s);
+    ss_status st = run_tile(h.val_dtype, h.c_dtype, g, h.tsmem, a, false, s);
     if (st || h.total_items == 0) return st;
   }
   void *fn;

@@ -12,14 +12,20 @@ namespace ss {
 // against 2.5 us of search latency in every block of the walk (N = 64:
 // 207 -> 203 us).
 __global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restrict__ indptr, int M, int tile,
-                                                        int tiles, int32_t *__restrict__ row_start,
+                                                        uint32_t inv_tile, int tiles, int32_t *__restrict__ row_start,
                                                         int *__restrict__ cnt, int ncnt) {
+  grid_dependents_launch();  // the walk may load its tiles; it waits for the rows
   const long long stride = (long long)gridDim.x * 256, i0 = blockIdx.x * 256ll + threadIdx.x;
+  // p / tile: the product with floor(2^32 / tile) is at most one short
+  auto tile_of = [&](int p) {
+    const int q = (int)__umulhi((uint32_t)p, inv_tile);
+    return p < 0 ? -1 : p - q * tile >= tile ? q + 1 : q;
+  };
   for (long long r0 = i0 * 4; r0 <= M; r0 += stride * 4) {
     int x[5];
-    x[0] = r0 > 0 ? __ldg(indptr + r0 - 1) / tile : -1;
+    x[0] = r0 > 0 ? tile_of(__ldg(indptr + r0 - 1)) : -1;
     #pragma unroll
-    for (int i = 0; i < 4; i++) x[i + 1] = r0 + i <= M ? __ldg(indptr + r0 + i) / tile : INT_MIN;
+    for (int i = 0; i < 4; i++) x[i + 1] = r0 + i <= M ? tile_of(__ldg(indptr + r0 + i)) : INT_MIN;
     #pragma unroll
     for (int i = 0; i < 4; i++)
       for (int t = max(x[i] + 1, 0); t <= min(x[i + 1], tiles - 1); t++) row_start[t] = (int)r0 + i;
@@ -63,7 +69,7 @@ TileGeom tile_geom(int N, int nnz, int dtype, int vmax, bool seg) {
   if (work <= half * most_piece) piece = ceil_div(work, half);
   else if (work > wave * most_piece && work <= 6 * wave * most_piece)
     piece = ceil_div(work, wave * ceil_div(work, wave * most_piece));
-  g.piece = (int)std::max(8LL, (piece + 3) / 4 * 4);
+  g.piece = (int)std::max(8LL, (piece + 7) / 8 * 8);  // odd strides of four words: no bank conflicts
   g.tile = NG * g.piece;
   g.tiles = std::max(1, ceil_div(nnz, g.tile));
   g.smem = (size_t)tile_smem(g.G, V * g.NV, g.piece).total * 4;
@@ -112,7 +118,8 @@ static void *tile_kernel(int val_dtype, int c_dtype, int G, int V, int NV, bool 
   return c_dtype == SS_F32 ? tile_kernel_f16_f32(G, V, NV, addc) : tile_kernel_f16(G, V, NV, addc);
 }
 
-ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, cudaStream_t s) {
+ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, bool after_rows,
+                   cudaStream_t s) {
   void *fn = tile_kernel(val_dtype, c_dtype, g.G, g.V, g.NV, a.accumulate != 0);
   if (!fn) return fail(SS_ERR_UNSUPPORTED_KNOBS, "no tile walk for G=%d V=%d NV=%d", g.G, g.V, g.NV);
   if (smem > 48 * 1024) {
@@ -120,7 +127,17 @@ ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, T
     if (e != cudaSuccess) return cuda_fail(e, "tile walk shared memory");
   }
   void *args[] = {&a};
-  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)(a.items * a.phases), 1, 1), dim3(TW_T, 1, 1), args, smem, s);
+  cudaLaunchAttribute overlap;
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(a.items * a.phases), 1, 1);
+  cfg.blockDim = dim3(TW_T, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = after_rows ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
   return e == cudaSuccess ? SS_OK : cuda_fail(e, "tile walk launch");
 }
 
@@ -145,11 +162,12 @@ ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
   a.keep_frac = l2_keep_fraction((size_t)c.K * c.N * dtype_size(c.val_dtype));
   const int ncnt = g.tiles * g.phases;
   const long long want = ((long long)c.M + 1024) / 1024;
-  tile_rows_kernel<<<(unsigned)std::min(want, (long long)sm_count() * 16), 256, 0, s>>>(c.indptr, c.M, g.tile, g.tiles,
+  tile_rows_kernel<<<(unsigned)std::min(want, (long long)sm_count() * 16), 256, 0, s>>>(c.indptr, c.M, g.tile,
+                                                                                      (uint32_t)((1ull << 32) / g.tile), g.tiles,
                                                                                       row_start, p.cnt, ncnt);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "tile rows launch");
-  return run_tile(c.val_dtype, c.c_dtype, g, g.smem, a, s);
+  return run_tile(c.val_dtype, c.c_dtype, g, g.smem, a, true, s);
 }
 
 // ---------------------------------------------------------------------

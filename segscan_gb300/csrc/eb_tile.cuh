@@ -48,7 +48,7 @@ struct __align__(16) TileProb {
   int *cnt;                  // [tiles * phases] arrivals per straddling row
   float *heads, *tails;      // [tiles * N] partials of a tile's first / last row
   int M, K, nnz;
-  int piece;       // nonzeros per group, a multiple of four
+  int piece;       // nonzeros per group, a multiple of eight
   uint32_t inv_piece;
   int item_begin;  // first block of this matrix (batched)
   int wide;        // columns and values may be loaded 16 bytes at a time
@@ -86,6 +86,12 @@ __host__ __device__ inline TileSmem tile_smem(int G, int E, int piece) {
 // e / piece for e below 2^16 and inv = ceil(2^32 / piece)
 __device__ __forceinline__ int piece_of(int e, uint32_t inv) { return (int)__umulhi((uint32_t)e, inv); }
 inline uint32_t inverse_of(int piece) { return (uint32_t)(((1ull << 32) + piece - 1) / piece); }
+
+// Waits for the kernels that this one was launched to overlap (programmatic
+// stream serialization); nothing to wait for in an ordinary launch.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel of the stream, if launched so, may start its blocks.
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <int V>
 __device__ __forceinline__ void store_smem(float *p, const float (&v)[V]) {
@@ -332,10 +338,10 @@ __device__ __forceinline__ int tile_walk(const TileProb &p, int N, int S, const 
         for (int i = 0; i < V; i++) acc[j][i] = fmaf(v, b[i], acc[j][i]);
       }
     }
-    const int out = hr ? end : 0;  // a row end after the first: stored here
+    const bool first = end != 0 && hr == 0; const int out = end != 0 && hr != 0;
     #pragma unroll
     for (int j = 0; j < NV; j++) {
-      if (end != out) store_smem<V>(shead + j * G * V, acc[j]);
+      if (first) store_smem<V>(shead + j * G * V, acc[j]);
       TC *d = (TC *)(Cj[j] + (uint64_t)(uint32_t)end * ldc);
       if (ADDC) {
         float x[V];
@@ -352,7 +358,7 @@ __device__ __forceinline__ int tile_walk(const TileProb &p, int N, int S, const 
         if (SLOW) comp[j][i] = end ? 0.f : comp[j][i];
       }
     }
-    hr = hr ? hr : end;
+    hr = first ? end : hr;
   };
   #pragma unroll 1
   for (int q = 0; q < S; q += 4) {
@@ -420,11 +426,36 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
 
   const int ts = tile * TILE;
   const int n = min(TILE, p.nnz - ts), te = ts + n;
+  // the tile's columns and values, on their way while the tile's rows are
+  // found (and, in a single launch, while the kernel that finds them runs)
+  constexpr int LOADS = 2;  // a tile is at most 2048 nonzeros
+  int c[LOADS][4];
+  float v[LOADS][4];
+  #pragma unroll
+  for (int k = 0; k < LOADS; k++) {
+    const int e = (tid + k * TW_T) * 4;
+    #pragma unroll
+    for (int i = 0; i < 4; i++) { c[k][i] = -1; v[k][i] = 1.f; }
+    if (e >= n) continue;
+    if (p.wide && e + 4 <= n) {
+      const uint4 x = ld_u128(p.cols + ts + e, strm);
+      c[k][0] = x.x; c[k][1] = x.y; c[k][2] = x.z; c[k][3] = x.w;
+      if (p.vals) load_vec<T, 4>((const T *)p.vals + ts + e, v[k], strm);
+    } else {
+      #pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (e + i >= n) continue;
+        c[k][i] = ld_idx(p.cols + ts + e + i, strm);
+        v[k][i] = load_val<T>((const T *)p.vals, (int64_t)ts + e + i, strm);
+      }
+    }
+  }
   // rows that start in the tile: [rlo, rhi)
   int rlo, rhi;
   if (p.row_start) {
-    rlo = __ldg(p.row_start + tile);
-    rhi = __ldg(p.row_start + tile + 1);
+    grid_dependency_wait();  // tile_rows_kernel has finished
+    rlo = __ldcg(p.row_start + tile);
+    rhi = __ldcg(p.row_start + tile + 1);
   } else if (tid < 64) {
     const int key = tid < 32 ? ts : te;
     const int r = tid < 32 ? (ts == 0 ? 0 : group_lower_bound(p.indptr, p.M, key, wl, 32, 0xffffffffu))
@@ -432,29 +463,19 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
     if (wl == 0) s_rows[tid >> 5] = r;
   }
   bool slow = false;
-  for (int e = tid * 4; e < TILE; e += TW_T * 4) {
-    int c[4];
-    float v[4] = {1.f, 1.f, 1.f, 1.f};
-    if (p.wide && e + 4 <= n) {
-      const uint4 x = ld_u128(p.cols + ts + e, strm);
-      c[0] = x.x; c[1] = x.y; c[2] = x.z; c[3] = x.w;
-      if (p.vals) load_vec<T, 4>((const T *)p.vals + ts + e, v, strm);
-    } else {
-      #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        c[i] = e + i < n ? ld_idx(p.cols + ts + e + i, strm) : -1;
-        if (p.vals) v[i] = e + i < n ? load_val<T>((const T *)p.vals, (int64_t)ts + e + i, strm) : 0.f;
-      }
-    }
+  #pragma unroll
+  for (int k = 0; k < LOADS; k++) {
+    const int e = (tid + k * TW_T) * 4;
+    if (e >= TILE) continue;
     #pragma unroll
     for (int i = 0; i < 4; i++)
-      if ((unsigned)c[i] >= (unsigned)p.K) {
-        c[i] = -1;
+      if ((unsigned)c[k][i] >= (unsigned)p.K) {
+        c[k][i] = -1;
         slow = true;
       }
     const int w = e + 4 * piece_of(e, p.inv_piece);
-    *reinterpret_cast<int4 *>(s_col + w) = make_int4(c[0], c[1], c[2], c[3]);
-    *reinterpret_cast<float4 *>(s_val + w) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<int4 *>(s_col + w) = make_int4(c[k][0], c[k][1], c[k][2], c[k][3]);
+    *reinterpret_cast<float4 *>(s_val + w) = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
     *reinterpret_cast<int4 *>(s_info + w) = make_int4(0, 0, 0, 0);
   }
   for (int i = tid; i < (TILE + 31) / 32; i += TW_T) s_kb[i] = 0;
@@ -612,6 +633,8 @@ struct TileGeom {
 // segment walk, whose rows stream instead of being gathered
 TileGeom tile_geom(int N, int nnz, int dtype, int vmax, bool seg = false);
 // Launches the walk of `a` (a.items * a.phases blocks, `smem` bytes each).
-ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, cudaStream_t s);
+// after_rows: right after tile_rows_kernel on the stream, which it overlaps.
+ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, bool after_rows,
+                   cudaStream_t s);
 
 }  // namespace ss

@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "rb_tile.cuh"
 
 namespace ss {
 
@@ -381,7 +382,53 @@ static ss_status launch_rb(bool pr, const SpmmCall &c, const RbGeom &g, cudaStre
   return SS_OK;
 }
 
-ss_status launch_rbsr(const SpmmCall &c, const RbGeom &g, cudaStream_t s) { return launch_rb(false, c, g, s); }
+// rbsr in groups of staged rows (rb_tile.cuh), whatever the tuple: a row's sum
+// does not depend on it.  Groups of fewer than eight lanes (a B row below 128
+// bytes) keep a row per team above: with many groups in a warp, each at its
+// own point of the staged walk, the warp runs them one after the other
+// (banded 300 K, N = 8: 19.1 us a row per team, 22.2 staged; Poisson 4096,
+// N = 16: 8.5 and 9.0).  Odd widths, whose lanes hold several single elements,
+// spill at a block of 1024 threads (N = 33: 26.7 and 30.7).  So does what a 32-bit row stride or the grid cannot
+// hold (N from 2^29, more than 65535 column phases).
+ss_status launch_rbsr(const SpmmCall &c, const RbGeom &geom, cudaStream_t s) {
+  if (c.M == 0 || c.N == 0) return SS_OK;
+  const TileGeom g = tile_geom(c.N, c.nnz, c.val_dtype,
+                               tile_vmax(c.B, dtype_size(c.val_dtype), c.C, dtype_size(c.c_dtype)));
+  if (g.G < 8 || g.V == 1 || c.N >= (1 << 29) || g.phases > 65535) return launch_rb(false, c, geom, s);
+  void *fn;
+  const bool addc = c.accumulate != 0;
+  if (c.val_dtype == SS_F32) fn = rb_tile_kernel_f32(g.G, g.V, g.NV, addc);
+  else if (c.val_dtype == SS_BF16)
+    fn = c.c_dtype == SS_F32 ? rb_tile_kernel_bf16_f32(g.G, g.V, g.NV, addc) : rb_tile_kernel_bf16(g.G, g.V, g.NV, addc);
+  else fn = c.c_dtype == SS_F32 ? rb_tile_kernel_f16_f32(g.G, g.V, g.NV, addc) : rb_tile_kernel_f16(g.G, g.V, g.NV, addc);
+  if (!fn) return fail(SS_ERR_UNSUPPORTED_KNOBS, "no rbsr kernel for G=%d V=%d NV=%d", g.G, g.V, g.NV);
+  RowArgs a;
+  a.indptr = c.indptr; a.cols = c.indices; a.vals = c.vals; a.B = c.B; a.C = c.C;
+  a.M = c.M; a.K = c.K; a.N = c.N; a.nnz = c.nnz; a.kahan = c.kahan_threshold;
+  a.keep_frac = l2_keep_fraction((size_t)c.K * c.N * dtype_size(c.val_dtype));
+  // rows that about fill a stage at the mean length, fewer where the groups of
+  // two blocks of 256 threads per SM would not all have some
+  const long long avg = std::max(1LL, ((long long)c.nnz + c.M - 1) / c.M);
+  const long long lanes = 2LL * TW_T * sm_count();
+  a.rows = (int)std::min((long long)g.G, std::max(1LL, ROW_CAP / avg));
+  while (a.rows > 1 && (long long)c.M * g.G * g.phases < lanes * a.rows) a.rows = (a.rows + 1) / 2;
+  // a block per SM (and column phase), as many threads as its rows have lanes
+  const long long units = ceil_div(c.M, a.rows), blocks = std::min((long long)sm_count(), units);
+  const long long per = (units + blocks - 1) / blocks;  // units per block
+  a.block_rows = (int)std::min((long long)c.M, per * a.rows);
+  const int most = addc ? 768 : 1024;
+  const int threads = (int)std::min((long long)most, (per * g.G + 31) / 32 * 32);
+  const int NG = threads / g.G;
+  const size_t smem = (size_t)3 * NG * (ROW_CAP + 4) * 4;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "rbsr shared memory");
+  }
+  void *args[] = {&a};
+  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)ceil_div(c.M, a.block_rows), (unsigned)g.phases, 1),
+                                   dim3(threads, 1, 1), args, smem, s);
+  return e == cudaSuccess ? SS_OK : cuda_fail(e, "rbsr launch");
+}
 ss_status launch_rbpr(const SpmmCall &c, const RbGeom &g, cudaStream_t s) { return launch_rb(true, c, g, s); }
 
 }  // namespace ss

@@ -357,11 +357,11 @@ void ss_mtx_free(ss_mtx *m);
  * m's chunk (thread_nz * 2^group_factor nonzeros); group_factor,
  * coarsen_factor and thread_per_block come from per_mat[0] (NULL = ebsr
  * defaults).  ss_batch_plan uploads the plan and synchronises the stream.
- * ss_spmm_batched then computes C[m] = A[m] * B[m] for every m in one
- * launch (after one memset of its counters; rows that straddle work items
- * are assembled inside that launch), or two when the batch has both
- * element-balanced matrices and row-balanced or long-chunk ones,
- * stream-ordered (it can be replayed from a captured CUDA graph).  Not in the reference. */
+ * ss_spmm_batched then computes C[m] = A[m] * B[m] for every m: one launch
+ * over the element-balanced matrices and a small one for the rows that
+ * straddle its work items, and one more (after a memset of its counters)
+ * when the batch has row-balanced or long-chunk matrices; stream-ordered (it
+ * can be replayed from a captured CUDA graph).  Not in the reference. */
 ss_status ss_batch_plan_size(int count, const ss_csr *mats, int N,
                              const ss_knobs *per_mat, size_t *host_bytes,
                              size_t *dev_bytes);

@@ -47,7 +47,7 @@ def features(A: api.CsrMatrix) -> dict:
 
 # bumped whenever the candidate list or the way candidates are timed
 # changes, so cached picks made the old way are measured again
-CANDIDATES_REV = 4
+CANDIDATES_REV = 5
 
 
 def signature(A: api.CsrMatrix, N: int, f: Optional[dict] = None) -> str:
@@ -58,29 +58,17 @@ def signature(A: api.CsrMatrix, N: int, f: Optional[dict] = None) -> str:
 
 
 def candidates(N: int, dtype: torch.dtype = torch.float32) -> list[tuple[str, dict]]:
-    """Strategy / knob candidates (README best static tuples, params.md grids,
-    and longer ebsr chunks, which suit the carry design).  16-bit storage also
-    tries 8-element vectors (16 bytes per lane, half the lanes per B row)."""
+    """Strategy / knob candidates (README best static tuples and params.md grids)."""
     c: list[tuple[str, dict]] = []
     for gf, denom in ((5, 8), (5, 16), (4, 4)):
         c.append(("ebpr", dict(group_factor=gf, tile_factor=5, block_denom=denom)))
     for gf, tf, denom in ((3, 3, 2), (2, 2, 1), (4, 4, 2)):
         c.append(("rbpr", dict(group_factor=gf, tile_factor=tf, block_denom=denom)))
-    vecs = (8, 4) if dtype in (torch.bfloat16, torch.float16) else (4,)
-    for vec in vecs:
-        lanes_gf = max(0, min(5, int(math.log2(max(1, N // vec)))))
-        for gf in sorted({lanes_gf, max(0, lanes_gf - 1)}):
-            for tnz in (2, 4, 8, 16, 32, 64):
-                for tpb in (128, 256, 512):
-                    c.append(("ebsr", dict(group_factor=gf, coarsen_factor=vec, thread_nz=tnz, block_denom=1,
-                                           thread_per_block=tpb)))
-    # one lane per group (the narrow walk) holding eight elements of a row
-    # each: the fastest layout at N = 8 (the group walk wins from N = 16 up)
-    if 8 <= N <= 16:
-        for tnz in (32, 64):
-            for tpb in (128, 256, 512):
-                c.append(("ebsr", dict(group_factor=0, coarsen_factor=8, thread_nz=tnz, block_denom=1,
-                                       thread_per_block=tpb)))
+    # every ebsr tuple with runs of up to 2048 nonzeros is the same tile walk
+    c.append(("ebsr", dict(thread_nz=2, block_denom=1)))
+    # the group walk with longer runs
+    lanes_gf = max(0, min(5, int(math.log2(max(1, N // 4)))))
+    c.append(("ebsr", dict(group_factor=lanes_gf, coarsen_factor=4, thread_nz=(4096 >> lanes_gf), block_denom=1)))
     # small blocks spread a small matrix's rows over more SMs
     for cf, tf in ((4, 5), (4, 6), (2, 5), (2, 6)):
         for tpb in (128, 256):

@@ -103,11 +103,12 @@ static ss_status batch_layout(int count, const ss_csr *mats, int N, const ss_kno
   h.mats_off = o; o += a256(sizeof(BatchMat) * (size_t)count);
   h.item_mat_off = o; o += a256(4 * (size_t)items);
   h.tprobs_off = o; o += a256(sizeof(TileProb) * (size_t)h.tile_count);
+  h.tfix_off = o; o += a256(sizeof(TileFix) * (size_t)h.tile_count);
   h.titem_off = o; o += a256(4 * (size_t)titems);
-  // arrival counts per (item, column tile) and (tile, column phase), then the
-  // work counters: one memset per step clears them
+  h.tspan_off = o; o += a256(8 * (size_t)titems);
+  // arrival counts per (item, column tile), then the work counters: one
+  // memset per step clears both
   h.rows_off = o; o += 4 * (size_t)items * (size_t)(h.tiles > 0 ? h.tiles : 1);
-  h.tcnt_off = o; o += 4 * (size_t)titems * (size_t)h.tphases;
   h.counter_off = o; o = a256(o + 4 * (size_t)(h.tiles > 0 ? h.tiles : 1));
   h.heads_off = o; o += a256(4 * (size_t)items * N);
   h.tails_off = o; o += a256(4 * (size_t)items * N);
@@ -122,7 +123,8 @@ static ss_status batch_layout(int count, const ss_csr *mats, int N, const ss_kno
 
 static size_t host_bytes_for(const BatchHeader &h) {
   return a256(sizeof(BatchHeader)) + a256(sizeof(BatchMat) * (size_t)h.count) + a256(4 * (size_t)h.total_items) +
-         a256(sizeof(TileProb) * (size_t)h.tile_count) + a256(4 * (size_t)h.tile_items);
+         a256(sizeof(TileProb) * (size_t)h.tile_count) + a256(sizeof(TileFix) * (size_t)h.tile_count) +
+         a256(4 * (size_t)h.tile_items);
 }
 
 // The sizes a plan may need, whatever the alignment of its operands.
@@ -188,19 +190,26 @@ ss_status ss_batch_plan_ex(int count, const ss_csr *mats, int N, const void *con
   for (int m = 0; m < count; m++)
     for (int c = 0; c < bm[m].num_chunks; c++) him[bm[m].item_begin + c] = m;
   TileProb *ht = (TileProb *)((char *)him + a256(4 * (size_t)h.total_items));
-  int32_t *hti = (int32_t *)((char *)ht + a256(sizeof(TileProb) * (size_t)h.tile_count));
+  TileFix *hf = (TileFix *)((char *)ht + a256(sizeof(TileProb) * (size_t)h.tile_count));
+  int32_t *hti = (int32_t *)((char *)hf + a256(sizeof(TileFix) * (size_t)h.tile_count));
+  std::vector<TileFix> tf((size_t)h.tile_count);
   char *db = (char *)dev_buf;
   for (int i = 0; i < h.tile_count; i++) {
     TileProb &p = tp[i];
     const int m = p.index;
     p.B = B[m];
     p.C = C[m];
-    p.cnt = (int *)(db + h.tcnt_off) + (size_t)p.item_begin * h.tphases;
+    p.span = (int2 *)(db + h.tspan_off) + p.item_begin;
     p.heads = (float *)(db + h.theads_off) + (size_t)p.item_begin * N;
     p.tails = (float *)(db + h.ttails_off) + (size_t)p.item_begin * N;
     const int end = i + 1 < h.tile_count ? tp[i + 1].item_begin : h.tile_items;
     for (int c = p.item_begin; c < end; c++) hti[c] = i;
+    TileFix &f = tf[(size_t)i];
+    memset(&f, 0, sizeof(f));
+    f.span = p.span; f.heads = p.heads; f.tails = p.tails; f.C = p.C;
+    f.M = p.M; f.tiles = end - p.item_begin; f.item_begin = p.item_begin;
   }
+  if (h.tile_count > 0) memcpy(hf, tf.data(), sizeof(TileFix) * (size_t)h.tile_count);
   if (h.tile_count > 0) memcpy(ht, tp.data(), sizeof(TileProb) * (size_t)h.tile_count);
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaMemcpyAsync((char *)dev_buf + h.mats_off, hm, sizeof(BatchMat) * (size_t)count,
@@ -209,6 +218,8 @@ ss_status ss_batch_plan_ex(int count, const ss_csr *mats, int N, const void *con
     e = cudaMemcpyAsync((char *)dev_buf + h.item_mat_off, him, 4 * (size_t)h.total_items, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && h.tile_count > 0)
     e = cudaMemcpyAsync(db + h.tprobs_off, ht, sizeof(TileProb) * (size_t)h.tile_count, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && h.tile_count > 0)
+    e = cudaMemcpyAsync(db + h.tfix_off, hf, sizeof(TileFix) * (size_t)h.tile_count, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && h.tile_items > 0)
     e = cudaMemcpyAsync(db + h.titem_off, hti, 4 * (size_t)h.tile_items, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the host buffer may be reused after return
@@ -235,9 +246,7 @@ ss_status ss_spmm_batched(const void *host_plan, void *dev_plan, void *stream) {
   if (h.total_items == 0 && h.tile_items == 0) return SS_OK;
   cudaStream_t s = (cudaStream_t)stream;
   char *plan = (char *)dev_plan;
-  // arrival counts and work counters (adjacent in the plan)
-  cudaError_t e = cudaMemsetAsync(plan + h.rows_off, 0, h.heads_off - h.rows_off, s);
-  if (e != cudaSuccess) return cuda_fail(e, "batched counter reset");
+  cudaError_t e;
   if (h.tile_items > 0) {
     TileArgs a;
     memset(&a, 0, sizeof(a));
@@ -254,8 +263,21 @@ ss_status ss_spmm_batched(const void *host_plan, void *dev_plan, void *stream) {
     g.V = h.tV;
     g.NV = h.tNV;
     ss_status st = run_tile(h.val_dtype, h.c_dtype, g, h.tsmem, a, false, s);
+    if (st == SS_OK && h.tile_items > h.tile_count) {  // some matrix has two tiles
+      FixArgs f;
+      memset(&f, 0, sizeof(f));
+      f.fixes = (const TileFix *)(plan + h.tfix_off);
+      f.item_prob = a.item_prob;
+      f.items = h.tile_items;
+      f.N = h.N;
+      f.reduce = SS_SUM;
+      st = run_fix(h.c_dtype, f, h.tV, s);
+    }
     if (st || h.total_items == 0) return st;
   }
+  // arrival counts and work counters (adjacent in the plan)
+  e = cudaMemsetAsync(plan + h.rows_off, 0, h.heads_off - h.rows_off, s);
+  if (e != cudaSuccess) return cuda_fail(e, "batched counter reset");
   void *fn;
   if (h.val_dtype == SS_F32) fn = batched_kernel_f32(h.V, h.NV);
   else if (h.val_dtype == SS_BF16) fn = batched_kernel_bf16(h.V, h.NV, h.c_dtype == SS_F32);

@@ -10,9 +10,9 @@
 // go to a persistent kernel: every group takes the next item from a device
 // counter (atomicAdd, no waiting on other groups) and walks it with the
 // ebsr chunk walk (eb_walk.cuh) against that matrix's arrays.  Straddling
-// rows go to the matrix's head/tail slots and the last of their tiles
-// or chunks to finish assembles them, so a step is one memset and one launch
-// (two when a batch has matrices of both kinds).
+// rows go to the matrix's head/tail slots; after the tile walk a small kernel
+// assembles them, in the persistent kernel the last of their chunks to
+// finish, after a memset of its counters.
 // Matrices without nonzeros are an empty tile, whose block writes the zeros.
 // The whole step is stream-ordered and can be captured in a graph.
 #pragma once
@@ -44,7 +44,7 @@ struct BatchHeader {
   size_t dev_bytes;
   // matrices walked by tiles
   int tile_count, tile_items, tG, tV, tNV, tphases;
-  size_t tsmem, tprobs_off, titem_off, tcnt_off, tstarts_off, theads_off, ttails_off;
+  size_t tsmem, tprobs_off, tfix_off, titem_off, tspan_off, theads_off, ttails_off;
 };
 
 template <typename T, typename TC, int V, int NV>

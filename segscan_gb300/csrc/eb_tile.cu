@@ -7,13 +7,10 @@
 namespace ss {
 
 // row_start[t] = first row that starts at or after nonzero t * tile_nz
-// (row_start[tiles] = M), one thread per row; also clears the arrival
-// counts, so the walk needs no memset of its own.  2 us on a million rows,
-// against 2.5 us of search latency in every block of the walk (N = 64:
-// 207 -> 203 us).
+// (row_start[tiles] = M), four rows a thread.  2 us on a million rows, against
+// 2.5 us of search latency in every block of the walk (N = 64: 207 -> 203 us).
 __global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restrict__ indptr, int M, int tile,
-                                                        uint32_t inv_tile, int tiles, int32_t *__restrict__ row_start,
-                                                        int *__restrict__ cnt, int ncnt) {
+                                                        uint32_t inv_tile, int tiles, int32_t *__restrict__ row_start) {
   grid_dependents_launch();  // the walk may load its tiles; it waits for the rows
   const long long stride = (long long)gridDim.x * 256, i0 = blockIdx.x * 256ll + threadIdx.x;
   // p / tile: the product with floor(2^32 / tile) is at most one short
@@ -31,7 +28,6 @@ __global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restric
       for (int t = max(x[i] + 1, 0); t <= min(x[i + 1], tiles - 1); t++) row_start[t] = (int)r0 + i;
   }
   if (i0 == 0) row_start[tiles] = M;
-  for (long long i = i0; i < ncnt; i += stride) cnt[i] = 0;
 }
 
 TileGeom tile_geom(int N, int nnz, int dtype, int vmax, bool seg) {
@@ -92,7 +88,7 @@ bool tile_fits(int N, int nnz, int dtype) {
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static size_t tile_ws(const TileGeom &g, int N) {
-  return align256((size_t)g.tiles * g.phases * 4) + align256((size_t)(g.tiles + 1) * 4) +
+  return align256((size_t)g.tiles * 8) + align256((size_t)(g.tiles + 1) * 4) +
          2 * (size_t)g.tiles * (size_t)N * sizeof(float);
 }
 
@@ -118,6 +114,88 @@ static void *tile_kernel(int val_dtype, int c_dtype, int G, int V, int NV, bool 
   return c_dtype == SS_F32 ? tile_kernel_f16_f32(G, V, NV, addc) : tile_kernel_f16(G, V, NV, addc);
 }
 
+// A launch whose blocks may start before the stream's last kernel has ended
+// (overlap): they wait for it where they need its results.
+static ss_status launch_overlapping(void *fn, void *arg, int blocks, size_t smem, bool overlap, cudaStream_t s,
+                                    const char *what) {
+  void *args[] = {arg};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks, 1, 1);
+  cfg.blockDim = dim3(TW_T, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+  return e == cudaSuccess ? SS_OK : cuda_fail(e, what);
+}
+
+// Rows that straddle tiles, a warp per tile: the row that starts in tile o
+// and goes on (span) is tail(o) + heads(o+1..last) in tile order with
+// compensation (or the maximum), plus the old row in accumulate mode, divided
+// by the segment's length for a mean; stored once.
+template <typename TC, int V>
+__global__ void __launch_bounds__(TW_T) fix_kernel(FixArgs a) {
+  grid_dependency_wait();  // the walk has finished
+  const int item = blockIdx.x * (TW_T / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (item >= a.items) return;
+  const TileFix f = a.item_prob ? a.fixes[__ldg(a.item_prob + item)] : a.f;
+  const int o = item - f.item_begin;
+  const int2 span = __ldcg(f.span + o);
+  const int r = span.x, l = span.y;
+  if ((unsigned)r >= (unsigned)f.M || l <= o || l >= f.tiles) return;
+  const bool is_max = a.reduce == SS_MAX, mean = a.reduce == SS_MEAN;
+  float len = 1.f;
+  if (mean) len = (float)(__ldcg(f.tcnt + o) + (l - o - 1) * f.tile_nz + __ldcg(f.hcnt + l));
+  const uint64_t strm = policy_stream();
+  constexpr int U = 4;  // heads in flight
+  for (int col = lane * V; col < a.N; col += 32 * V) {
+    float acc[V], comp[V];
+    load_slot<V>(f.tails + (int64_t)o * a.N + col, acc);
+    #pragma unroll
+    for (int i = 0; i < V; i++) comp[i] = 0.f;
+    for (int k = o + 1; k <= l; k += U) {
+      float x[U][V];
+      #pragma unroll
+      for (int u = 0; u < U; u++) load_slot<V>(f.heads + (int64_t)min(k + u, l) * a.N + col, x[u]);
+      #pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (k + u > l) break;
+        #pragma unroll
+        for (int i = 0; i < V; i++) {
+          if (is_max) acc[i] = fmaxf(acc[i], x[u][i]);
+          else kahan_add(acc[i], comp[i], x[u][i]);
+        }
+      }
+    }
+    TC *d = (TC *)f.C + (int64_t)r * a.N + col;
+    if (a.accumulate) {
+      float old[V];
+      load_old<TC, V>(d, old);
+      #pragma unroll
+      for (int i = 0; i < V; i++) acc[i] += old[i];
+    }
+    if (mean) {
+      #pragma unroll
+      for (int i = 0; i < V; i++) acc[i] = acc[i] / len;
+    }
+    store_vec<TC, V>(d, acc, strm);
+  }
+}
+
+template <typename TC>
+static void *fix_ptr(int V) {
+  return V >= 4 ? (void *)fix_kernel<TC, 4> : V == 2 ? (void *)fix_kernel<TC, 2> : (void *)fix_kernel<TC, 1>;
+}
+
+ss_status run_fix(int c_dtype, FixArgs &a, int V, cudaStream_t s) {
+  void *fn = c_dtype == SS_F32 ? fix_ptr<float>(V) : c_dtype == SS_BF16 ? fix_ptr<__nv_bfloat16>(V) : fix_ptr<__half>(V);
+  return launch_overlapping(fn, &a, ceil_div(a.items, TW_T / 32), 0, true, s, "straddling rows launch");
+}
+
 ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, bool after_rows,
                    cudaStream_t s) {
   void *fn = tile_kernel(val_dtype, c_dtype, g.G, g.V, g.NV, a.accumulate != 0);
@@ -126,19 +204,7 @@ ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, T
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "tile walk shared memory");
   }
-  void *args[] = {&a};
-  cudaLaunchAttribute overlap;
-  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  overlap.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(a.items * a.phases), 1, 1);
-  cfg.blockDim = dim3(TW_T, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &overlap;
-  cfg.numAttrs = after_rows ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
-  return e == cudaSuccess ? SS_OK : cuda_fail(e, "tile walk launch");
+  return launch_overlapping(fn, &a, a.items * a.phases, smem, after_rows, s, "tile walk launch");
 }
 
 ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
@@ -152,7 +218,7 @@ ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
   p.piece = g.piece; p.inv_piece = inverse_of(g.piece);
   p.wide = (((uintptr_t)c.indices | (uintptr_t)c.vals) & 15u) == 0;
   char *w = (char *)ws;
-  p.cnt = (int *)w; w += align256((size_t)g.tiles * g.phases * 4);
+  p.span = (int2 *)w; w += align256((size_t)g.tiles * 8);
   int32_t *row_start = (int32_t *)w; w += align256((size_t)(g.tiles + 1) * 4);
   p.row_start = row_start;
   p.heads = (float *)w;
@@ -160,21 +226,27 @@ ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
   a.items = g.tiles; a.phases = g.phases;
   a.N = c.N; a.accumulate = c.accumulate; a.kahan = c.kahan_threshold;
   a.keep_frac = l2_keep_fraction((size_t)c.K * c.N * dtype_size(c.val_dtype));
-  const int ncnt = g.tiles * g.phases;
   const long long want = ((long long)c.M + 1024) / 1024;
   tile_rows_kernel<<<(unsigned)std::min(want, (long long)sm_count() * 16), 256, 0, s>>>(c.indptr, c.M, g.tile,
                                                                                       (uint32_t)((1ull << 32) / g.tile), g.tiles,
-                                                                                      row_start, p.cnt, ncnt);
+                                                                                      row_start);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "tile rows launch");
-  return run_tile(c.val_dtype, c.c_dtype, g, g.smem, a, true, s);
+  ss_status st = run_tile(c.val_dtype, c.c_dtype, g, g.smem, a, true, s);
+  if (st || g.tiles == 1) return st;  // one tile: no row straddles
+  FixArgs f;
+  memset(&f, 0, sizeof(f));
+  f.f.span = p.span; f.f.heads = p.heads; f.f.tails = p.tails; f.f.C = c.C;
+  f.f.M = c.M; f.f.tiles = g.tiles; f.f.tile_nz = g.tile;
+  f.items = g.tiles; f.N = c.N; f.accumulate = c.accumulate; f.reduce = SS_SUM;
+  return run_fix(c.c_dtype, f, g.V, s);
 }
 
 // ---------------------------------------------------------------------
 // segment_coo
 // ---------------------------------------------------------------------
 static size_t seg_tile_ws(const TileGeom &g, int N) {
-  return align256((size_t)g.tiles * g.phases * 4) + align256((size_t)2 * g.tiles * 4) +
+  return align256((size_t)g.tiles * 8) + align256((size_t)2 * g.tiles * 4) +
          2 * (size_t)g.tiles * (size_t)N * sizeof(float);
 }
 
@@ -204,8 +276,7 @@ ss_status launch_seg_tile(const SegCall &c, bool kahan, void *ws, cudaStream_t s
   a.M = c.dst_len; a.nnz = c.nnz; a.N = c.N; a.piece = g.piece; a.inv_piece = inverse_of(g.piece); a.tiles = g.tiles; a.phases = g.phases;
   a.reduce = c.reduce; a.kahan = kahan;
   char *w = (char *)ws;
-  const size_t cnt_bytes = align256((size_t)g.tiles * g.phases * 4);
-  a.cnt = (int *)w; w += cnt_bytes;
+  a.span = (int2 *)w; w += align256((size_t)g.tiles * 8);
   a.hcnt = (int *)w;
   a.tcnt = a.hcnt + g.tiles; w += align256((size_t)2 * g.tiles * 4);
   a.heads = (float *)w;
@@ -214,13 +285,18 @@ ss_status launch_seg_tile(const SegCall &c, bool kahan, void *ws, cudaStream_t s
              : c.src_dtype == SS_BF16 ? seg_tile_kernel_bf16(g.G, g.V, g.NV, c.accumulate != 0)
                                       : seg_tile_kernel_f16(g.G, g.V, g.NV, c.accumulate != 0);
   if (!fn) return fail(SS_ERR_UNSUPPORTED_KNOBS, "no segment tile walk for G=%d V=%d NV=%d", g.G, g.V, g.NV);
-  cudaError_t e = cudaMemsetAsync(a.cnt, 0, (size_t)g.tiles * g.phases * 4, s);
-  if (e != cudaSuccess) return cuda_fail(e, "segment arrival counts");
   const int NG = TW_T / g.G;
   const size_t smem = ((size_t)NG * (g.piece + 4) + 2 * (size_t)TW_T * g.V * g.NV + ceil_div(g.tile, 32)) * 4;
   void *args[] = {&a};
-  e = cudaLaunchKernel(fn, dim3((unsigned)(g.tiles * g.phases), 1, 1), dim3(TW_T, 1, 1), args, smem, s);
-  return e == cudaSuccess ? SS_OK : cuda_fail(e, "segment tile walk launch");
+  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)(g.tiles * g.phases), 1, 1), dim3(TW_T, 1, 1), args, smem, s);
+  if (e != cudaSuccess) return cuda_fail(e, "segment tile walk launch");
+  if (g.tiles == 1) return SS_OK;
+  FixArgs f;
+  memset(&f, 0, sizeof(f));
+  f.f.span = a.span; f.f.heads = a.heads; f.f.tails = a.tails; f.f.hcnt = a.hcnt; f.f.tcnt = a.tcnt;
+  f.f.C = c.dst; f.f.M = c.dst_len; f.f.tiles = g.tiles; f.f.tile_nz = g.tile;
+  f.items = g.tiles; f.N = c.N; f.accumulate = c.accumulate; f.reduce = c.reduce;
+  return run_fix(SS_F32, f, g.V, s);
 }
 
 }  // namespace ss

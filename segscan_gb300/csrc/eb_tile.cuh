@@ -20,8 +20,11 @@
 //  * a group's first row end may belong to a row that an earlier group
 //    started: it goes to shared memory with every group's last partial, and
 //    the pieces of a row are added in order after the walk;
-//  * rows that straddle tiles go through one head and one tail slot per tile
-//    and the last participant stores them (tile_arrive), as in carry_arrive.
+//  * rows that straddle tiles leave their parts in one head and one tail slot
+//    per tile; a small kernel, launched to overlap the walk's end, adds them
+//    up (fix_kernel in eb_tile.cu).  Counting the tiles in with atomics and
+//    letting the last one add cost every block 5 to 12 K of its 60 K cycles,
+//    with nothing else of the block in flight.
 // Nonzeros of rows longer than kahan_threshold are summed with compensation:
 // warps that hold any take a second instantiation of the walk, which also
 // skips columns outside [0, K).
@@ -45,7 +48,7 @@ struct __align__(16) TileProb {
   const void *B;
   void *C;
   const int32_t *row_start;  // [tiles + 1] first row starting at or after each tile, or null: searched
-  int *cnt;                  // [tiles * phases] arrivals per straddling row
+  int2 *span;                // [tiles] row that starts in the tile and goes on (or -1), its last tile
   float *heads, *tails;      // [tiles * N] partials of a tile's first / last row
   int M, K, nnz;
   int piece;       // nonzeros per group, a multiple of eight
@@ -254,42 +257,6 @@ __device__ __forceinline__ void tile_store(const TileProb &p, int N, int row, co
   }
 }
 
-// Counts this tile in for row r, which straddles tiles o..l; the last tile to
-// arrive sums tail(o) + heads(o+1..l) in tile order with compensation and
-// stores the row, so the result does not depend on which one is last.
-template <typename TC, int G, int V, int NV, bool ADDC>
-__device__ __forceinline__ void tile_arrive(const TileProb &p, int N, int tile_nz, int r, int lane,
-                                            unsigned mask, int phase, int phases, int col0, const bool (&act)[NV],
-                                            uint64_t pol) {
-  const int s = __ldg(p.indptr + r), e = __ldg(p.indptr + r + 1);
-  if ((unsigned)s >= (unsigned)p.nnz || (unsigned)(e - 1) >= (unsigned)p.nnz) return;  // malformed indptr
-  const int o = s / tile_nz, l = (e - 1) / tile_nz;
-  __threadfence();  // this lane's slot stores are visible before the count moves
-  __syncwarp(mask);
-  int last = 0;
-  if (lane == 0) last = atomicAdd(p.cnt + (size_t)o * phases + phase, 1) == l - o;
-  last = __shfl_sync(mask, last, 0, G);
-  if (!last) return;
-  __threadfence();  // every other participant's slot is visible now
-  float acc[NV][V];
-  clear<V, NV>(acc);
-  #pragma unroll
-  for (int j = 0; j < NV; j++) {
-    if (!act[j]) continue;
-    const int64_t col = col0 + j * G * V;
-    float comp[V], x[V];
-    load_slot<V>(p.tails + (int64_t)o * N + col, acc[j]);
-    #pragma unroll
-    for (int i = 0; i < V; i++) comp[i] = 0.f;
-    for (int k = o + 1; k <= l; k++) {
-      load_slot<V>(p.heads + (int64_t)k * N + col, x);
-      #pragma unroll
-      for (int i = 0; i < V; i++) kahan_add(acc[j][i], comp[i], x[i]);
-    }
-  }
-  tile_store<TC, G, V, NV, ADDC>(p, N, r, acc, col0, act, pol);
-}
-
 // One group's piece: S nonzeros from its staged columns, values and row-end
 // marks.  The first row end goes to shead (its row + 1 is returned, 0 when
 // the piece has none), what follows the last one to stail, the others to C.
@@ -409,6 +376,7 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
   }
   __syncthreads();
   const TileProb &p = *reinterpret_cast<const TileProb *>(smem);
+  grid_dependents_launch();  // fix_kernel, which waits for this grid
   const int S = p.piece, TILE = NG * S;
   const TileSmem L = tile_smem(G, E, S);
   int32_t *s_col = smem + L.col, *s_info = smem + L.info;
@@ -539,9 +507,11 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
   }
   const int gb = g * (S + 4);
   float *shead = s_head + g * COLS + lane * V, *stail = s_tail + g * COLS + lane * V;
+  // accumulating into 16 bits is rare: one instantiation, the one that fits all
+  constexpr bool FAST = !(ADDC && sizeof(TC) == 2);
   int hr;
-  if (!slow)
-    hr = tile_walk<T, TC, G, V, NV, false, ADDC>(p, a.N, S, s_col + gb, s_val + gb, s_info + gb, s_kb, g * S, shead,
+  if (FAST && !slow)
+    hr = tile_walk<T, TC, G, V, NV, !FAST, ADDC>(p, a.N, S, s_col + gb, s_val + gb, s_info + gb, s_kb, g * S, shead,
                                            stail, lane, col0, act, keep, strm);
   else
     hr = tile_walk<T, TC, G, V, NV, true, ADDC>(p, a.N, S, s_col + gb, s_val + gb, s_info + gb, s_kb, g * S, shead,
@@ -583,18 +553,21 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
     chain(s, g, true, acc);
     if (s < 0 && has_head) {  // the row that entered the tile ends
       to_slot(p.heads, acc);
-      tile_arrive<TC, G, V, NV, ADDC>(p, a.N, TILE, rlo - 1, lane, mask, phase, a.phases, col0, act, strm);
     } else {
       tile_store<TC, G, V, NV, ADDC>(p, a.N, hr - 1, acc, col0, act, strm);
     }
   }
-  if (g == 0 && te < p.nnz && __ldg(p.indptr + rhi) > te) {  // the last row goes on
-    const int s = prev_end(NG);
-    chain(s, NG, false, acc);
-    const bool whole = s < 0 && has_head;  // the tile lies inside one row
-    to_slot(whole ? p.heads : p.tails, acc);
-    tile_arrive<TC, G, V, NV, ADDC>(p, a.N, TILE, whole ? rlo - 1 : rhi - 1, lane, mask, phase, a.phases, col0, act,
-                                    strm);
+  if (g == 0) {
+    const int next = te < p.nnz ? __ldg(p.indptr + rhi) : te;  // where the tile's last row ends
+    int2 span = make_int2(-1, 0);
+    if (next > te) {  // it goes on
+      const int s = prev_end(NG);
+      chain(s, NG, false, acc);
+      const bool whole = s < 0 && has_head;  // the tile lies inside one row
+      to_slot(whole ? p.heads : p.tails, acc);
+      if (!whole) span = make_int2(rhi - 1, (next - 1) / TILE);
+    }
+    if (lane == 0) p.span[tile] = span;  // every phase writes the same
   }
 }
 
@@ -634,6 +607,22 @@ struct TileGeom {
 TileGeom tile_geom(int N, int nnz, int dtype, int vmax, bool seg = false);
 // Launches the walk of `a` (a.items * a.phases blocks, `smem` bytes each).
 // after_rows: right after tile_rows_kernel on the stream, which it overlaps.
+// What fix_kernel needs of one matrix (or segment reduction).
+struct TileFix {
+  const int2 *span;
+  const float *heads, *tails;
+  const int *hcnt, *tcnt;  // segment means
+  void *C;
+  int M, tiles, item_begin, tile_nz;
+};
+struct FixArgs {
+  TileFix f;               // single launch
+  const TileFix *fixes;    // batched: the matrices and the matrix of each tile
+  const int32_t *item_prob;
+  int items, N, accumulate, reduce;
+};
+// Launched right after the walk.
+ss_status run_fix(int c_dtype, FixArgs &a, int vmax, cudaStream_t s);
 ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, bool after_rows,
                    cudaStream_t s);
 

@@ -8,8 +8,7 @@
 // element whose successor has another id is marked with its id + 1 (the
 // index itself says where segments end, so no search), a group's first
 // segment end and its last partial go to shared memory and are combined in
-// order, and segments that straddle tiles are stored by the last tile to
-// arrive.  The rows of src stream in order, eight ahead where the registers
+// order, and segments that straddle tiles are put together by fix_kernel.  The rows of src stream in order, eight ahead where the registers
 // allow.  Sum, max and mean; sums of every element with compensation where
 // the tuple's chunk is longer than the threshold.
 //
@@ -24,7 +23,7 @@ struct SegTileArgs {
   const void *src;
   const int32_t *index;
   float *dst;
-  int *cnt;             // [tiles * phases] arrivals per straddling segment
+  int2 *span;           // [tiles] segment that starts in the tile and goes on (or -1), its last tile
   int *hcnt, *tcnt;     // [tiles] elements of a tile's first / last segment (means)
   float *heads, *tails;  // [tiles * N] their partials
   int M, nnz, N, piece, tiles, phases, reduce, kahan;  // piece: elements per group
@@ -70,43 +69,6 @@ __device__ __forceinline__ void seg_store(const SegTileArgs &a, int row, float (
     }
     store_vec<float, V>(dst + j * G * V, x, pol);
   }
-}
-
-// This tile's part of segment r (tiles o..l) is in its slot: the last tile to
-// arrive combines tail(o) and heads(o+1..l) in order and stores the segment.
-template <int G, int V, int NV, bool ADDC>
-__device__ __forceinline__ void seg_arrive(const SegTileArgs &a, int r, int o, int l, int tile_nz, int lane,
-                                           unsigned mask, int phase, int col0, const bool (&act)[NV], uint64_t pol) {
-  if ((unsigned)r >= (unsigned)a.M) return;  // every participant sees the same r: none counts
-  __threadfence();
-  __syncwarp(mask);
-  int last = 0;
-  if (lane == 0) last = atomicAdd(a.cnt + (size_t)o * a.phases + phase, 1) == l - o;
-  last = __shfl_sync(mask, last, 0, G);
-  if (!last) return;
-  __threadfence();
-  int count = 1;
-  if (a.reduce == SS_MEAN) count = __ldcg(a.tcnt + o) + (l - o - 1) * tile_nz + __ldcg(a.hcnt + l);
-  float acc[NV][V];
-  clear<V, NV>(acc);
-  #pragma unroll
-  for (int j = 0; j < NV; j++) {
-    if (!act[j]) continue;
-    const int64_t col = col0 + j * G * V;
-    float comp[V], x[V];
-    load_slot<V>(a.tails + (int64_t)o * a.N + col, acc[j]);
-    #pragma unroll
-    for (int i = 0; i < V; i++) comp[i] = 0.f;
-    for (int k = o + 1; k <= l; k++) {
-      load_slot<V>(a.heads + (int64_t)k * a.N + col, x);
-      #pragma unroll
-      for (int i = 0; i < V; i++) {
-        if (a.reduce == SS_MAX) acc[j][i] = fmaxf(acc[j][i], x[i]);
-        else kahan_add(acc[j][i], comp[i], x[i]);
-      }
-    }
-  }
-  seg_store<G, V, NV, ADDC>(a, r, acc, count, col0, act, pol);
 }
 
 // One group's piece of m elements, from element p0 of the tile.  Marks: id + 1
@@ -216,7 +178,7 @@ template <typename T, int G, int V, int NV, bool ADDC>
 __global__ void __launch_bounds__(TW_T, (ADDC || V * NV > 4 ? 3 : 4)) seg_tile_kernel(SegTileArgs a) {
   constexpr int NG = TW_T / G, E = V * NV, COLS = G * E, EW = (NG + 31) / 32;
   extern __shared__ __align__(16) int32_t smem[];
-  __shared__ int s_own[2];  // owner tile of the segment that enters, last tile of the one that leaves
+  __shared__ int s_last;  // last tile of the segment that leaves this one
   __shared__ uint32_t s_ends[EW];
   __shared__ int s_hn[NG], s_tn[NG];
   const int S = a.piece, TILE = NG * S;
@@ -237,6 +199,7 @@ __global__ void __launch_bounds__(TW_T, (ADDC || V * NV > 4 ? 3 : 4)) seg_tile_k
   #pragma unroll
   for (int j = 0; j < NV; j++) act[j] = col0 + j * G * V < a.N;
   if (tid < EW) s_ends[tid] = 0;
+  grid_dependents_launch();  // fix_kernel, which waits for this grid
 
   // segment ends, and the empty segments after each of them
   auto zero_gap = [&](int lo, int hi) {  // the whole warp; lo, hi uniform
@@ -276,21 +239,7 @@ __global__ void __launch_bounds__(TW_T, (ADDC || V * NV > 4 ? 3 : 4)) seg_tile_k
   const int r_in = __ldg(a.index + ts), r_out = __ldg(a.index + te - 1);
   const bool has_head = ts > 0 && __ldg(a.index + ts - 1) == r_in;
   const bool more = te < a.nnz && __ldg(a.index + te) == r_out;
-  if (tid < 32 && has_head) {
-    // nearest tile before this one whose first id is below r: r starts there,
-    // or with the tile after it when that tile's last id is not r
-    int o = 0;
-    for (int base = tile - 1; base >= 0; base -= 32) {
-      const int j = base - wl;
-      const unsigned m = __ballot_sync(0xffffffffu, j < 0 || __ldg(a.index + (int64_t)j * TILE) < r_in);
-      if (m) {
-        const int k = base - (__ffs(m) - 1);
-        o = k < 0 ? 0 : __ldg(a.index + (int64_t)(k + 1) * TILE - 1) == r_in ? k : k + 1;
-        break;
-      }
-    }
-    if (wl == 0) s_own[0] = o;
-  } else if (tid >= 32 && tid < 64 && more) {
+  if (tid >= 32 && tid < 64 && more) {
     // last tile whose first id is still r
     int l = a.tiles - 1;
     for (int base = tile + 1; base < a.tiles; base += 32) {
@@ -301,7 +250,7 @@ __global__ void __launch_bounds__(TW_T, (ADDC || V * NV > 4 ? 3 : 4)) seg_tile_k
         break;
       }
     }
-    if (wl == 0) s_own[1] = l;
+    if (wl == 0) s_last = l;
   }
   __syncthreads();
   const int m = min(max(n - g * S, 0), S);
@@ -372,17 +321,20 @@ __global__ void __launch_bounds__(TW_T, (ADDC || V * NV > 4 ? 3 : 4)) seg_tile_k
     chain(s, g, true, acc, count);
     if (s < 0 && has_head) {  // the segment that entered the tile ends
       to_slot(a.heads, a.hcnt, acc, count);
-      seg_arrive<G, V, NV, ADDC>(a, r_in, s_own[0], tile, TILE, lane, mask, phase, col0, act, strm);
     } else if (hr > 0) {
       seg_store<G, V, NV, ADDC>(a, hr - 1, acc, count, col0, act, strm);
     }
   }
-  if (g == 0 && more) {  // the last segment goes on
-    const int s = prev_end(NG);
-    chain(s, NG, false, acc, count);
-    const bool whole = s < 0 && has_head;  // the tile lies inside one segment
-    to_slot(whole ? a.heads : a.tails, whole ? a.hcnt : a.tcnt, acc, count);
-    seg_arrive<G, V, NV, ADDC>(a, r_out, whole ? s_own[0] : tile, s_own[1], TILE, lane, mask, phase, col0, act, strm);
+  if (g == 0) {
+    int2 span = make_int2(-1, 0);
+    if (more) {  // the last segment goes on
+      const int s = prev_end(NG);
+      chain(s, NG, false, acc, count);
+      const bool whole = s < 0 && has_head;  // the tile lies inside one segment
+      to_slot(whole ? a.heads : a.tails, whole ? a.hcnt : a.tcnt, acc, count);
+      if (!whole) span = make_int2(r_out, s_last);
+    }
+    if (lane == 0) a.span[tile] = span;  // every phase writes the same
   }
 }
 

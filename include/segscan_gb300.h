@@ -183,6 +183,22 @@ ss_status ss_spmm_ebsr(const ss_csr *A, int N, const void *B, void *C,
                        int c_dtype, int accumulate, const ss_knobs *knobs,
                        void *ws, size_t ws_bytes, void *stream);
 
+/* C = A * B with A's values read through a permutation: the value of A's
+ * nonzero q is values[perm[q]] (SS_F32 / SS_BF16 / SS_F16, widened), so A^T
+ * times a gradient needs no gathered copy of the values.  A holds the pattern
+ * (its values are ignored, value_dtype SS_F32); B is FP32, C is SS_F32, SS_BF16
+ * or SS_F16.  The tile walk only: SS_ERR_UNSUPPORTED_KNOBS (also from the
+ * size query) where ss_spmm_ebsr would take the group walk.  Not in the
+ * reference. */
+ss_status ss_spmm_permuted_workspace_size(const ss_csr *A, int N,
+                                          const ss_knobs *knobs,
+                                          size_t *bytes);
+ss_status ss_spmm_permuted(const ss_csr *A, const int32_t *perm,
+                           const void *values, int value_dtype, int N,
+                           const float *B, void *C, int c_dtype,
+                           const ss_knobs *knobs, void *ws, size_t ws_bytes,
+                           void *stream);
+
 /* The ebsr SpMM without a workspace argument, for callers that cannot
  * allocate device memory: a host that only holds buffers handed to it by
  * another allocator, or a loop where cudaMalloc's blocking, device

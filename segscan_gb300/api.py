@@ -215,6 +215,37 @@ def spmm(A: CsrMatrix, B: torch.Tensor, strategy: str = "ebsr", knobs: Optional[
     return out
 
 
+@_allocates_on_launch_stream
+def spmm_permuted(A: CsrMatrix, perm: torch.Tensor, values: torch.Tensor, B: torch.Tensor,
+                  knobs: Optional[SsKnobs] = None, out_dtype: Optional[torch.dtype] = None,
+                  stream=None) -> Optional[torch.Tensor]:
+    """C = A(values[perm]) @ B with FP32 B, the values read in place (as A^T @ dC
+    reads A's values); the bits of gathering values.float() first and calling
+    spmm(..., "ebsr").  None where the tuple or the size takes ebsr's group
+    walk, which reads its own values only."""
+    if B.dim() != 2 or B.shape[0] != A.ncol:
+        raise ValueError(f"B must be [{A.ncol}, N], got {tuple(B.shape)}")
+    _need_cuda("B", B, torch.float32)
+    _need_cuda("perm", perm, torch.int32)
+    _need_cuda("values", values)
+    if perm.numel() != A.nnz or values.numel() != A.nnz:
+        raise ValueError(f"perm ({perm.numel()}), values ({values.numel()}) and A ({A.nnz}) differ in nonzeros")
+    N, cdt = int(B.shape[1]), out_dtype or torch.float32
+    d = A.with_values(None).descr()
+    kp = ctypes.byref(knobs) if knobs is not None else None
+    n = ctypes.c_size_t()
+    rc = _lib.load().ss_spmm_permuted_workspace_size(ctypes.byref(d), N, kp, ctypes.byref(n))
+    if rc == _lib.Status.UNSUPPORTED_KNOBS:
+        return None
+    _lib.check(rc)
+    out = _output((A.nrow, N), cdt, B.device)
+    ws = _workspace(int(n.value), B.device)
+    wp, wn = _aligned(ws)
+    _lib.call("ss_spmm_permuted", ctypes.byref(d), _ptr(perm), _ptr(values), int(dtype_code(values.dtype)), N, _ptr(B),
+              _ptr(out), int(dtype_code(cdt)), kp, wp, wn, _stream(stream))
+    return out
+
+
 class _Plan:
     """A bound call: run() validates and makes one C call whose last argument
     is the stream handle; capture() records it into a CUDA graph."""

@@ -9,7 +9,8 @@ Backward:
   by the stable counting-sort transpose once per pattern and cached;
   one of them, or N above the fused walk's width:
   dA.vals = SDDMM(dC, B)            (ss_sddmm: dot of dC row i with B row k)
-  dB      = A^T @ dC                (the forward kernels on A^T)
+  dB      = A^T @ dC                (the forward kernels on A^T; ebsr reads
+                                     A's values through the permutation)
 Values stored in BF16/FP16 get FP32 gradients cast back to their dtype;
 dB is computed in FP32 (A^T values widened to FP32) and rounded to B's dtype
 by the ebsr walk's own stores (other strategies: a cast after).
@@ -68,6 +69,9 @@ class SpMMFunction(torch.autograd.Function):
             d_values = api.sddmm(A, dC, B.contiguous()).to(values.dtype)
         if ctx.needs_input_grad[1]:
             AT, perm = pattern.transposed()
+            if ctx.bw_strategy == "ebsr":  # A's values read through the permutation, no gathered copy
+                d_B = api.spmm_permuted(AT, perm, values.contiguous(), dC, ctx.bw_knobs, B.dtype)
+        if ctx.needs_input_grad[1] and d_B is None:
             t_vals = api.gather_values(values.float().contiguous(), perm)
             AT_v = AT.with_values(t_vals)
             if ctx.bw_strategy == "ebsr" and B.dtype != torch.float32:

@@ -468,6 +468,71 @@ ss_status ss_spmm(int strategy, const ss_csr *A, int N, const void *B, void *C, 
   return strategy == SS_RBSR ? launch_rbsr(c, rg, s) : launch_rbpr(c, rg, s);
 }
 
+// Whether the tile walk serves this call (it reads values through the
+// permutation; no other kernel does).
+static ss_status permuted_call(const ss_csr *A, int N, const ss_knobs *knobs, ss_knobs &tmp, const ss_knobs **k) {
+  *k = knobs_or_default(SS_EBSR, N, knobs, tmp);
+  if (!*k) return SS_ERR_INVALID_ARG;
+  ss_status st = check_csr(A, N);
+  if (st) return st;
+  if (A->value_dtype != SS_F32) return fail(SS_ERR_INVALID_ARG, "the pattern's value_dtype must be SS_F32 (B's type)");
+  EbGeom g;
+  st = geom_sr(A->nrow, A->nnz, N, SS_F32, 4, **k, g);
+  if (st) return st;
+  if (A->nnz > 0 && N > 0 && !takes_tile(**k, N, A->nnz, SS_F32))
+    return fail(SS_ERR_UNSUPPORTED_KNOBS, "permuted values need the tile walk (runs of up to 2048 nonzeros)");
+  return SS_OK;
+}
+
+ss_status ss_spmm_permuted_workspace_size(const ss_csr *A, int N, const ss_knobs *knobs, size_t *bytes) {
+  if (!bytes) return fail(SS_ERR_INVALID_ARG, "bytes is null");
+  ss_knobs tmp;
+  const ss_knobs *k;
+  ss_status st = permuted_call(A, N, knobs, tmp, &k);
+  if (st) return st;
+  *bytes = A->nnz > 0 && N > 0 ? tile_workspace_bytes(N, A->nnz, SS_F32) : 0;
+  return SS_OK;
+}
+
+ss_status ss_spmm_permuted(const ss_csr *A, const int32_t *perm, const void *values, int value_dtype, int N,
+                           const float *B, void *C, int c_dtype, const ss_knobs *knobs, void *ws, size_t ws_bytes,
+                           void *stream) {
+  ss::NvtxRange nvtx_range("ss_spmm");
+  ss_knobs tmp;
+  const ss_knobs *k;
+  ss_status st = permuted_call(A, N, knobs, tmp, &k);
+  if (st) return st;
+  if (value_dtype < SS_F32 || value_dtype > SS_F16) return fail(SS_ERR_INVALID_ARG, "value_dtype %d unknown", value_dtype);
+  if (A->nnz > 0 && (!perm || !values)) return fail(SS_ERR_INVALID_ARG, "perm or values is null");
+  if (((uintptr_t)perm % 4) || ((uintptr_t)values % dtype_size(value_dtype)))
+    return fail(SS_ERR_ALIGNMENT, "pointer not aligned to its element size");
+  ss_csr P = *A;
+  P.values = nullptr;
+  SpmmCall c;
+  st = make_spmm_call(SS_EBSR, &P, N, B, C, c_dtype, 0, *k, c);
+  if (st) return st;
+  c.vals = values;
+  c.perm = perm;
+  c.perm_dtype = value_dtype;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (c.M == 0 || c.N == 0) return SS_OK;
+  EbGeom g;
+  st = geom_sr(c.M, c.nnz, N, SS_F32, 4, *k, g);
+  if (st) return st;
+  st = check_vec_alignment(B, C, 4, dtype_size(c_dtype), g.cs.V);
+  if (st) return st;
+  if (c.nnz == 0 || hypersparse(c.nnz, c.M)) {
+    cudaError_t e = cudaMemsetAsync(C, 0, (size_t)c.M * c.N * dtype_size(c.c_dtype), s);
+    if (e != cudaSuccess) return cuda_fail(e, "zero C");
+    if (c.nnz == 0) return SS_OK;
+    c.accumulate = 1;
+  }
+  const size_t need = tile_workspace_bytes(N, c.nnz, SS_F32);
+  if (ws_bytes < need || !ws || ((uintptr_t)ws % 256))
+    return fail(SS_ERR_WORKSPACE, "workspace needs %zu bytes (256-byte aligned), got %zu", need, ws_bytes);
+  return launch_ebsr_tile(c, ws, s);
+}
+
 ss_status ss_spmm_ebpr(const ss_csr *A, int N, const void *B, void *C, int c_dtype, int accumulate,
                        const ss_knobs *knobs, void *ws, size_t ws_bytes, void *stream) {
   return ss_spmm(SS_EBPR, A, N, B, C, c_dtype, accumulate, knobs, ws, ws_bytes, stream);

@@ -215,6 +215,7 @@ ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
   TileProb &p = a.p;
   p.indptr = c.indptr; p.cols = c.indices; p.vals = c.vals; p.B = c.B; p.C = c.C;
   p.M = c.M; p.K = c.K; p.nnz = c.nnz;
+  p.perm = c.perm; p.perm_dtype = c.perm_dtype;
   p.piece = g.piece; p.inv_piece = inverse_of(g.piece);
   p.wide = (((uintptr_t)c.indices | (uintptr_t)c.vals) & 15u) == 0;
   char *w = (char *)ws;

@@ -47,6 +47,7 @@ struct __align__(16) TileProb {
   const void *vals;  // null = ones
   const void *B;
   void *C;
+  const int32_t *perm;       // value of nonzero q is vals[perm[q]] in type perm_dtype, or null: vals[q]
   const int32_t *row_start;  // [tiles + 1] first row starting at or after each tile, or null: searched
   int2 *span;                // [tiles] row that starts in the tile and goes on (or -1), its last tile
   float *heads, *tails;      // [tiles * N] partials of a tile's first / last row
@@ -56,6 +57,7 @@ struct __align__(16) TileProb {
   int item_begin;  // first block of this matrix (batched)
   int wide;        // columns and values may be loaded 16 bytes at a time
   int index;       // host: the matrix's place in its batch
+  int perm_dtype;
 };
 
 struct TileArgs {
@@ -405,7 +407,18 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
     #pragma unroll
     for (int i = 0; i < 4; i++) { c[k][i] = -1; v[k][i] = 1.f; }
     if (e >= n) continue;
-    if (p.wide && e + 4 <= n) {
+    if (sizeof(T) == 4 && p.perm) {  // values in another order and type
+      #pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (e + i >= n) continue;
+        c[k][i] = ld_idx(p.cols + ts + e + i, strm);
+        const int q = ld_idx(p.perm + ts + e + i, strm);
+        v[k][i] = (unsigned)q >= (unsigned)p.nnz ? 0.f
+                  : p.perm_dtype == SS_F32       ? load_val<float>((const float *)p.vals, q, keep)
+                  : p.perm_dtype == SS_BF16      ? load_val<__nv_bfloat16>((const __nv_bfloat16 *)p.vals, q, keep)
+                                                 : load_val<__half>((const __half *)p.vals, q, keep);
+      }
+    } else if (p.wide && e + 4 <= n) {
       const uint4 x = ld_u128(p.cols + ts + e, strm);
       c[k][0] = x.x; c[k][1] = x.y; c[k][2] = x.z; c[k][3] = x.w;
       if (p.vals) load_vec<T, 4>((const T *)p.vals + ts + e, v[k], strm);

@@ -35,6 +35,8 @@ struct SpmmCall {
   int c_dtype;       // SS_F32 or val_dtype
   int accumulate;
   int kahan_threshold;
+  const int32_t *perm = nullptr;  // tile walk: the value of nonzero q is vals[perm[q]],
+  int perm_dtype = SS_F32;        // of this type
 };
 
 // One segment_coo problem after argument checks.

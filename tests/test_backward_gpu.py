@@ -249,3 +249,33 @@ def test_fused_backward_wide_refused(cuda):
     with pytest.raises(SegscanError):
         api.spmm_backward(AT, perm, A.values, torch.zeros((100, N), device="cuda"),
                           torch.zeros((80, N), device="cuda"))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_values_through_the_permutation(cuda, dtype):
+    """spmm_permuted gives the bits of gathering the values first: every width class, output type,
+    order of the permutation and alignment, an almost empty matrix, an empty one; tuples of the
+    group walk are refused."""
+    from segscan_gb300 import api
+    rng = np.random.default_rng(3)
+    for csr in (synth.powerlaw(9000, 7000, 2.1, 1, 3000, seed=2), synth.poisson(5000, 4000, 0.2, seed=3),
+                synth.Csr(6, 5, np.zeros(7, np.int32), np.zeros(0, np.int32), np.zeros(0, np.float32))):
+        A = dev_csr(csr, values=False)
+        perm = torch.from_numpy(rng.permutation(csr.nnz).astype(np.int32)).cuda()
+        vals = torch.from_numpy(csr.values).cuda().to(dtype)
+        if csr.nnz:
+            shifted = torch.empty(csr.nnz + 1, dtype=torch.int32, device="cuda")
+            shifted[1:] = perm
+        gathered = vals.float()[perm.long()].contiguous()
+        for N in (1, 4, 6, 33, 64, 100):
+            B = torch.from_numpy(synth.dense(csr.ncol, N, seed=N)).cuda()
+            for out_dtype in (torch.float32, torch.bfloat16):
+                ref = api.spmm(A.with_values(gathered), B, "ebsr", out_dtype=out_dtype)
+                assert torch.equal(ref, api.spmm_permuted(A, perm, vals, B, out_dtype=out_dtype))
+            if csr.nnz:
+                assert torch.equal(api.spmm(A.with_values(gathered), B, "ebsr"),
+                                   api.spmm_permuted(A, shifted[1:], vals, B))
+    assert api.spmm_permuted(dev_csr(synth.poisson(50, 40, 3.0, seed=1), values=False),
+                             torch.zeros(synth.poisson(50, 40, 3.0, seed=1).nnz, dtype=torch.int32, device="cuda"),
+                             torch.zeros(synth.poisson(50, 40, 3.0, seed=1).nnz, device="cuda", dtype=dtype),
+                             torch.zeros(40, 64, device="cuda"), api.make_knobs("ebsr", 64, thread_nz=256)) is None

@@ -8,7 +8,7 @@ namespace ss {
 
 // row_start[t] = first row that starts at or after nonzero t * tile_nz
 // (row_start[tiles] = M), four rows a thread.  2 us on a million rows, against
-// 2.5 us of search latency in every block of the walk (N = 64: 207 -> 203 us).
+// 2.5 us of search latency in every wave of the walk (N = 64: 207 -> 203 us).
 __global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restrict__ indptr, int M, int tile,
                                                         uint32_t inv_tile, int tiles, int32_t *__restrict__ row_start) {
   grid_dependents_launch();  // the walk may load its tiles; it waits for the rows
@@ -221,19 +221,25 @@ ss_status launch_ebsr_tile(const SpmmCall &c, void *ws, cudaStream_t s) {
   char *w = (char *)ws;
   p.span = (int2 *)w; w += align256((size_t)g.tiles * 8);
   int32_t *row_start = (int32_t *)w; w += align256((size_t)(g.tiles + 1) * 4);
-  p.row_start = row_start;
+  // No more blocks than are resident at once: each searches its own rows and
+  // the launch is saved (Poisson 12 a row, N = 64: 1 K rows at N = 16 6.97 ->
+  // 6.06 us, 40 K rows 23.5 -> 20.4 us).  With more waves every one pays for
+  // the search (80 K rows 29.1 -> 30.0 us, 1 M rows at N = 16 110 -> 116 us).
+  const bool searched = (long long)g.tiles * g.phases <= 4LL * sm_count();
+  p.row_start = searched ? nullptr : row_start;
   p.heads = (float *)w;
   p.tails = p.heads + (size_t)g.tiles * c.N;
   a.items = g.tiles; a.phases = g.phases;
   a.N = c.N; a.accumulate = c.accumulate; a.kahan = c.kahan_threshold;
   a.keep_frac = l2_keep_fraction((size_t)c.K * c.N * dtype_size(c.val_dtype));
-  const long long want = ((long long)c.M + 1024) / 1024;
-  tile_rows_kernel<<<(unsigned)std::min(want, (long long)sm_count() * 16), 256, 0, s>>>(c.indptr, c.M, g.tile,
-                                                                                      (uint32_t)((1ull << 32) / g.tile), g.tiles,
-                                                                                      row_start);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "tile rows launch");
-  ss_status st = run_tile(c.val_dtype, c.c_dtype, g, g.smem, a, true, s);
+  if (!searched) {
+    const long long want = ((long long)c.M + 1024) / 1024;
+    tile_rows_kernel<<<(unsigned)std::min(want, (long long)sm_count() * 16), 256, 0, s>>>(
+        c.indptr, c.M, g.tile, (uint32_t)((1ull << 32) / g.tile), g.tiles, row_start);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "tile rows launch");
+  }
+  ss_status st = run_tile(c.val_dtype, c.c_dtype, g, g.smem, a, !searched, s);
   if (st || g.tiles == 1) return st;  // one tile: no row straddles
   FixArgs f;
   memset(&f, 0, sizeof(f));

@@ -160,3 +160,11 @@ def test_scratch_of_the_group_walk_is_still_accepted(cuda):
     C64, absC = oracle64(csr, Bd.cpu().numpy())
     for C in (ref, got):
         assert np.all(np.abs(C.double().cpu().numpy() - C64) <= 1e-5 * absC + 1e-30)
+
+
+@pytest.mark.parametrize("N,nnz", [(4, 1_100_000), (4, 1_400_000), (256, 140_000), (256, 170_000)])
+def test_rows_searched_and_listed(cuda, N, nnz):
+    """On both sides of one wave of blocks: below it each block searches its rows, above it a kernel lists them."""
+    csr = shaped(mixed(nnz), 6000)
+    B = synth.dense(csr.ncol, N, seed=N)
+    check(csr, B, dev_csr(csr, torch.float32), torch.from_numpy(B).cuda(), torch.float32, torch.float32, f"nnz={nnz}")

@@ -167,4 +167,6 @@ def check(status: int) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(load(), name)(*args))
+    rc = getattr(_lib or load(), name)(*args)
+    if rc:
+        check(rc)

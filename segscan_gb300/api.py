@@ -35,6 +35,9 @@ SEG_STRATEGIES = {"pr": SegStrategy.PR, "sr": SegStrategy.SR}
 REDUCES = {"sum": Reduce.SUM, "max": Reduce.MAX, "mean": Reduce.MEAN}
 
 
+_F32 = Dtype.F32
+
+
 def dtype_code(t: torch.dtype) -> Dtype:
     try:
         return _DTYPE_OF[t]
@@ -48,8 +51,12 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 def _stream(stream) -> int:
     if stream is None:
-        stream = torch.cuda.current_stream()
+        # (given the index, torch does not look for the device)
+        return torch.cuda.current_stream(torch.cuda.current_device()).cuda_stream
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
+
+
+_NO_CONTEXT = contextlib.nullcontext()
 
 
 def _on(stream):
@@ -57,7 +64,7 @@ def _on(stream):
     do when the caller passed none, so the current stream is the launch
     stream already)."""
     if stream is None:
-        return contextlib.nullcontext()
+        return _NO_CONTEXT
     if not isinstance(stream, torch.cuda.Stream):
         handle = stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
         if handle == torch.cuda.current_stream().cuda_stream:
@@ -130,16 +137,19 @@ class CsrMatrix:
     def descr(self) -> SsCsr:
         # the C ABI sees only pointers and sizes: tensors shorter than the
         # sizes claim would be read past their ends on the device
-        if self.indptr.numel() != self.nrow + 1:
-            raise ValueError(f"indptr must hold nrow + 1 = {self.nrow + 1} entries, got {self.indptr.numel()}")
-        if self.values is not None and self.values.numel() != self.nnz:
-            raise ValueError(f"values must hold nnz = {self.nnz} entries (as indices), got {self.values.numel()}")
-        _need_cuda("indptr", self.indptr, torch.int32)
-        _need_cuda("indices", self.indices, torch.int32)
-        if self.values is not None:
-            _need_cuda("values", self.values)
-        return SsCsr(self.nrow, self.ncol, self.nnz, _ptr(self.indptr), _ptr(self.indices),
-                     _ptr(self.values), int(dtype_code(self.dtype)))
+        indptr, indices, values = self.indptr, self.indices, self.values
+        nnz = indices.numel()
+        if indptr.numel() != self.nrow + 1:
+            raise ValueError(f"indptr must hold nrow + 1 = {self.nrow + 1} entries, got {indptr.numel()}")
+        if values is not None and values.numel() != nnz:
+            raise ValueError(f"values must hold nnz = {nnz} entries (as indices), got {values.numel()}")
+        _need_cuda("indptr", indptr, torch.int32)
+        _need_cuda("indices", indices, torch.int32)
+        if values is None:
+            return SsCsr(self.nrow, self.ncol, nnz, indptr.data_ptr(), indices.data_ptr(), None, _F32)
+        _need_cuda("values", values)
+        return SsCsr(self.nrow, self.ncol, nnz, indptr.data_ptr(), indices.data_ptr(), values.data_ptr(),
+                     dtype_code(values.dtype))
 
 
 def default_knobs(strategy: str, N: int = 64) -> SsKnobs:
@@ -182,11 +192,14 @@ def _aligned(ws: Optional[torch.Tensor]) -> tuple[Optional[int], int]:
 
 
 def spmm_workspace_size(A: CsrMatrix, N: int, strategy: str, knobs: Optional[SsKnobs] = None) -> int:
+    return _spmm_workspace_size(A.descr(), N, strategy, knobs)
+
+
+def _spmm_workspace_size(d: SsCsr, N: int, strategy: str, knobs: Optional[SsKnobs]) -> int:
     n = ctypes.c_size_t()
-    d = A.descr()
-    _lib.call("ss_spmm_workspace_size", int(STRATEGIES[strategy]), ctypes.byref(d), N,
+    _lib.call("ss_spmm_workspace_size", STRATEGIES[strategy], ctypes.byref(d), N,
               ctypes.byref(knobs) if knobs is not None else None, ctypes.byref(n))
-    return int(n.value)
+    return n.value
 
 
 @_allocates_on_launch_stream
@@ -202,16 +215,16 @@ def spmm(A: CsrMatrix, B: torch.Tensor, strategy: str = "ebsr", knobs: Optional[
     cdt = out_dtype or (out.dtype if out is not None else torch.float32)
     if out is None:
         out = _output((A.nrow, N), cdt, B.device)
-    _need_cuda("out", out, cdt)
-    if tuple(out.shape) != (A.nrow, N):
-        raise ValueError(f"out must be [{A.nrow}, {N}]")
+    else:
+        _need_cuda("out", out, cdt)
+        if tuple(out.shape) != (A.nrow, N):
+            raise ValueError(f"out must be [{A.nrow}, {N}]")
     d = A.descr()
-    kp = ctypes.byref(knobs) if knobs is not None else None
     if workspace is None:
-        workspace = _workspace(spmm_workspace_size(A, N, strategy, knobs), B.device)
+        workspace = _workspace(_spmm_workspace_size(d, N, strategy, knobs), B.device)
     wp, wn = _aligned(workspace)
-    _lib.call("ss_spmm", int(STRATEGIES[strategy]), ctypes.byref(d), N, _ptr(B), _ptr(out),
-              int(dtype_code(cdt)), int(bool(accumulate)), kp, wp, wn, _stream(stream))
+    _lib.call("ss_spmm", STRATEGIES[strategy], ctypes.byref(d), N, B.data_ptr(), out.data_ptr(), dtype_code(cdt),
+              1 if accumulate else 0, ctypes.byref(knobs) if knobs is not None else None, wp, wn, _stream(stream))
     return out
 
 
@@ -387,7 +400,8 @@ def segment(src: torch.Tensor, index: torch.Tensor, dst_len: int, reduce: str = 
     _need_cuda("index", index, torch.int32)
     if out is None:
         out = _output((dst_len, N), torch.float32, src.device)
-    _need_cuda("out", out, torch.float32)
+    else:
+        _need_cuda("out", out, torch.float32)
     ws = workspace if workspace is not None else _workspace(segment_workspace_size(nnz, N, strategy, knobs),
                                                              src.device)
     wp, wn = _aligned(ws)

@@ -21,6 +21,8 @@
 // fixed butterfly (butterfly_sum); dB is summed in position order, with
 // Kahan compensation when the row is longer than the threshold, so dB has
 // the bits of the row-balanced sequential SpMM (rbsr) on A^T.  FP32 math.
+#include <algorithm>
+
 #include "common.cuh"
 #include "eb_common.cuh"
 #include "internal.h"
@@ -271,18 +273,29 @@ extern "C" ss_status ss_spmm_backward(const ss_csr *AT, const int32_t *perm, con
   a.t_indptr = AT->indptr; a.t_indices = AT->indices; a.perm = perm; a.vals = values;
   a.dC = dC; a.B = B; a.dB = dB; a.dvals = dvals;
   a.lanes = lanes; a.log2_lanes = ilog2(lanes);
-  // shares of about nnz / (eight blocks per SM's groups) positions, at least 64
   const int threads = 256;
   const long long groups_per_block = threads / lanes;
-  const long long target = (long long)sm_count() * 8 * groups_per_block;
-  long long chunk = ((long long)nnz + target - 1) / target;
-  if (chunk < 64) chunk = 64;
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0);
+  if (e != cudaSuccess) return cuda_fail(e, "fused backward occupancy");
+  const long long wave = (long long)sm_count() * std::max(per_sm, 1) * groups_per_block;
+  // Shares of whole rows, equal in nonzeros, that fill whole waves of resident
+  // blocks: one, or several of about 450 nonzeros a group, which even out the
+  // long rows (1.9 M power-law rows, N = 128: one wave 1041, two 1023, four
+  // 1011 us; Poisson 200 K rows, N = 64: one 169, two 178, four 196 us; one
+  // and a quarter waves cost 40 %).  Down to two batches a group where a wave
+  // is not filled: the serial chain is what is left there (Poisson 4 K rows,
+  // N = 64: shares of 64 29.0, 16 15.1, 8 15.2 us; power-law 60 K rows,
+  // N = 32: 40.5, 22.0, 20.2 us).
+  const long long waves = std::max(1LL, (nnz + wave * 225) / (wave * 450));
+  long long chunk = ((long long)nnz + wave * waves - 1) / (wave * waves);
+  chunk = std::max(chunk, 2LL * BWD_U);
   long long groups = ((long long)nnz + chunk - 1) / chunk;
   if (groups < 1) groups = 1;
   a.chunk = (int)chunk;
   a.groups = (int)groups;
   const long long blocks = (groups + groups_per_block - 1) / groups_per_block;
   void *args[] = {&a};
-  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(threads), args, 0, (cudaStream_t)stream);
+  e = cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(threads), args, 0, (cudaStream_t)stream);
   return e == cudaSuccess ? SS_OK : cuda_fail(e, "fused backward launch");
 }

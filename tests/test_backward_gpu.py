@@ -279,3 +279,23 @@ def test_values_through_the_permutation(cuda, dtype):
                              torch.zeros(synth.poisson(50, 40, 3.0, seed=1).nnz, dtype=torch.int32, device="cuda"),
                              torch.zeros(synth.poisson(50, 40, 3.0, seed=1).nnz, device="cuda", dtype=dtype),
                              torch.zeros(40, 64, device="cuda"), api.make_knobs("ebsr", 64, thread_nz=256)) is None
+
+
+@pytest.mark.parametrize("N", [4, 47, 64, 128])
+@pytest.mark.parametrize("ncol,per", [(1, 1), (1, 7), (1, 8), (1, 9), (3, 17), (40, 3), (5000, 12), (300_000, 3)])
+def test_fused_backward_shares(cuda, N, ncol, per):
+    """Shares of eight nonzeros up to whole waves, rows of A^T longer than a share: FP64 within 1e-5 of
+    sum|terms| and, for dB, the bits of rbsr on A^T."""
+    from segscan_gb300 import api
+    csr = synth.poisson(max(2 * per, ncol), ncol, float(min(per, ncol)), seed=per)
+    A = dev_csr(csr)
+    B, dC = synth.dense(csr.ncol, N, seed=1), synth.dense(csr.nrow, N, seed=2)
+    dCd = torch.from_numpy(dC).cuda()
+    AT, perm = api.transpose(A)
+    dvals, dB = api.spmm_backward(AT, perm, A.values, dCd, torch.from_numpy(B).cuda())
+    ref = api.spmm(AT.with_values(api.gather_values(A.values, perm)), dCd, "rbsr",
+                   knobs=api.make_knobs("rbsr", N, coarsen_factor=4, tile_factor=7))
+    torch.cuda.synchronize()
+    assert torch.equal(dB, ref)
+    dv64, dvabs = oracle_lib.sddmm_f64(csr.indptr, csr.indices, dC, B)
+    check_close(dvals.cpu().numpy(), dv64, dvabs, 1e-5, 1e-5, f"dvals N={N}")

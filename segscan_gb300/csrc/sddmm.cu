@@ -18,13 +18,15 @@
 //    is issued, compile-time lane masks.
 // B rows are gathered with an evict-last L2 policy; dC rows too when dC fits
 // in half the L2, else evict-first (they are read once, row after row).
+#include <algorithm>
+
 #include "common.cuh"
 #include "eb_common.cuh"
 #include "internal.h"
 
 namespace ss {
 
-constexpr int SDDMM_CHUNK = 128;  // nonzeros per team chunk
+constexpr int SDDMM_CHUNK = 192;  // nonzeros per team chunk, about (128 to 256: no difference)
 constexpr int SDDMM_U = 8;        // nonzeros per step, sub-warp teams
 constexpr int SDDMM_WU = 4;       // nonzeros per step, whole-warp teams
 
@@ -43,7 +45,7 @@ __global__ void __launch_bounds__(256) sddmm_rows_kernel(int M, int K, int N, in
                                                          const int32_t *__restrict__ indptr,
                                                          const int32_t *__restrict__ cols, const float *__restrict__ dC,
                                                          const T *__restrict__ B, float *__restrict__ out, int lanes,
-                                                         int log2_lanes, int dc_stream) {
+                                                         int log2_lanes, int dc_stream, int chunk_nz) {
   const int tid = threadIdx.x;
   const int lane = tid & (lanes - 1);
   const int team = (blockIdx.x * blockDim.x + tid) >> log2_lanes;
@@ -52,9 +54,9 @@ __global__ void __launch_bounds__(256) sddmm_rows_kernel(int M, int K, int N, in
   const unsigned mask = lanes >= 32 ? 0xffffffffu : (((1u << lanes) - 1u) << (wl & ~(unsigned)(lanes - 1)));
   const uint64_t keep = policy_keep(1.0f), strm = policy_stream();
   const uint64_t dc_pol = dc_stream ? strm : keep;
-  const int nchunks = (nnz + SDDMM_CHUNK - 1) / SDDMM_CHUNK;
+  const int nchunks = (nnz - 1) / chunk_nz + 1;
   for (int chunk = team; chunk < nchunks; chunk += teams) {
-    const int cs = chunk * SDDMM_CHUNK, ce = min(cs + SDDMM_CHUNK, nnz);
+    const int cs = chunk * chunk_nz, ce = cs + min(chunk_nz, nnz - cs);
     int row = row_search(indptr, 1, M, cs);
     int next = __ldg(indptr + min(row + 1, M));
     for (int p0 = cs; p0 < ce; p0 += SDDMM_U) {
@@ -100,6 +102,7 @@ struct SddmmArgs {
   const float *dC;  // [M x N]
   const void *B;    // [K x N], the values' storage type
   float *out;       // [nnz]
+  int chunk;        // nonzeros per team chunk (last: 7 % slower at N = 128 with the pointers moved)
 };
 
 // Whole-warp teams: lane masks and shuffle widths are compile-time
@@ -116,9 +119,9 @@ __global__ void __launch_bounds__(256, 4) sddmm_warp_kernel(SddmmArgs a) {
   const uint64_t keep = policy_keep(1.0f), strm = policy_stream();
   const uint64_t dc_pol = a.dc_stream ? strm : keep;
   const T *__restrict__ B = (const T *)a.B;
-  const int nchunks = (a.nnz + SDDMM_CHUNK - 1) / SDDMM_CHUNK;
+  const int nchunks = (a.nnz - 1) / a.chunk + 1;
   for (int chunk = team; chunk < nchunks; chunk += teams) {
-    const int cs = chunk * SDDMM_CHUNK, ce = min(cs + SDDMM_CHUNK, a.nnz);
+    const int cs = chunk * a.chunk, ce = cs + min(a.chunk, a.nnz - cs);
     // the row holding cs (the last row starting at or before it), then the
     // window: lane l holds indptr[wb + l]
     int wb = max(min(group_lower_bound(a.indptr, a.M, cs + 1, lane, L, mask), a.M) - 1, 0);
@@ -230,29 +233,37 @@ extern "C" ss_status ss_sddmm(const ss_csr *A, int N, const float *dC, const voi
   void *fn = A->value_dtype == SS_F32 ? sddmm_ptr<float>(V, warp)
              : A->value_dtype == SS_BF16 ? sddmm_ptr<__nv_bfloat16>(V, warp) : sddmm_ptr<__half>(V, warp);
   const int threads = 256;
-  const long long teams_needed = ((long long)nnz + SDDMM_CHUNK - 1) / SDDMM_CHUNK;
-  long long blocks = (teams_needed * lanes + threads - 1) / threads;
-  if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-  if (blocks < 1) blocks = 1;
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0);
+  if (e != cudaSuccess) return cuda_fail(e, "sddmm occupancy");
+  // Chunks that fill whole waves of resident teams, about SDDMM_CHUNK
+  // nonzeros each or what one wave leaves: with fixed chunks of 128 a small
+  // matrix left SMs idle (Poisson 4 K rows, N = 64 43 -> 6 us; power-law 60 K
+  // rows, N = 32 52 -> 9.3 us) and a larger one ended in a part wave (700 K
+  // rows BF16 N = 64 194 -> 147 us).
+  const long long wave = (long long)sm_count() * std::max(per_sm, 1) * (threads / lanes);
+  const long long waves = std::max(1LL, (nnz + wave * SDDMM_CHUNK / 2) / (wave * SDDMM_CHUNK));
+  long long chunk = ((long long)nnz + wave * waves - 1) / (wave * waves);
+  chunk = std::max((chunk + SDDMM_WU - 1) / SDDMM_WU * SDDMM_WU, (long long)SDDMM_U);
+  const long long blocks = (((long long)nnz + chunk - 1) / chunk * lanes + threads - 1) / threads;
   // dC is read row after row, each row's reuse served by L1: when it is
   // larger than half the L2, its lines are marked evict-first so that they
   // do not push out the gathered B rows; a smaller dC is kept like B
   const int dc_stream = (long long)A->nrow * N * 4 > l2_bytes() / 2;
-  cudaError_t e;
   if (warp) {
     SddmmArgs a;
     a.M = A->nrow; a.K = A->ncol; a.N = N; a.nnz = nnz;
     a.slices = ceil_div(N, lanes * V);
     a.indptr = A->indptr; a.cols = A->indices; a.dC = dC; a.B = B; a.out = dvals;
-    a.dc_stream = dc_stream;
+    a.dc_stream = dc_stream; a.chunk = (int)chunk;
     void *args[] = {&a};
     e = cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(threads), args, 0, (cudaStream_t)stream);
   } else {
     int log2_lanes = ilog2(lanes);
     int M = A->nrow, K = A->ncol, Nn = N, nz = nnz;
     const int32_t *ip = A->indptr, *ix = A->indices;
-    int dcs = dc_stream;
-    void *args[] = {&M, &K, &Nn, &nz, &ip, &ix, &dC, &B, &dvals, &lanes, &log2_lanes, &dcs};
+    int dcs = dc_stream, cnz = (int)chunk;
+    void *args[] = {&M, &K, &Nn, &nz, &ip, &ix, &dC, &B, &dvals, &lanes, &log2_lanes, &dcs, &cnz};
     e = cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(threads), args, 0, (cudaStream_t)stream);
   }
   return e == cudaSuccess ? SS_OK : cuda_fail(e, "sddmm launch");

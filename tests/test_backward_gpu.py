@@ -299,3 +299,17 @@ def test_fused_backward_shares(cuda, N, ncol, per):
     assert torch.equal(dB, ref)
     dv64, dvabs = oracle_lib.sddmm_f64(csr.indptr, csr.indices, dC, B)
     check_close(dvals.cpu().numpy(), dv64, dvabs, 1e-5, 1e-5, f"dvals N={N}")
+
+
+@pytest.mark.parametrize("N", [3, 4, 64, 128])
+@pytest.mark.parametrize("rows,mean", [(1, 1), (1, 7), (1, 9), (3, 17), (5000, 12), (60_000, 12)])
+def test_sddmm_chunks(cuda, N, rows, mean):
+    """Chunks of eight nonzeros up to whole waves, against FP64 within 1e-5 of sum|terms|."""
+    from segscan_gb300 import api
+    csr = synth.poisson(rows, max(32, rows // 2), float(mean), seed=mean)
+    A = dev_csr(csr)
+    B, dC = synth.dense(csr.ncol, N, seed=1), synth.dense(csr.nrow, N, seed=2)
+    got = api.sddmm(A, torch.from_numpy(dC).cuda(), torch.from_numpy(B).cuda())
+    torch.cuda.synchronize()
+    want, terms = oracle_lib.sddmm_f64(csr.indptr, csr.indices, dC, B)
+    check_close(got.cpu().numpy(), want, terms, 1e-5, 1e-5, f"sddmm N={N} rows={rows}")

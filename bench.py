@@ -358,7 +358,7 @@ def extra_batched(dev, N=64, count=512, headline=None):
     res["plain_fp32_per_matrix_ms"] = plain_ms
     res["plain_chunk_target"] = plain_target
     # the same per-matrix launches replayed from one CUDA graph (no host
-    # overhead left: what remains is one memset and one walk per matrix)
+    # overhead left: what remains is the walk's kernels per matrix)
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):
         plain()
@@ -561,9 +561,14 @@ def run_ours(args):
     C = torch.empty((Ah.nrow, N), dtype=torch.float32, device=dev)
     work = S.kernels.workspace(Ad, N)
     stream = torch.cuda.current_stream(dev)
-    # ebsr: one walk launch (straddling rows assembled inside it, after a
-    # memset of the arrival counts); ebpr: scan + fix-up; row-balanced: one
+    # ebsr with runs of up to 2048 nonzeros: the tiles' first rows (above one
+    # wave of 1024-nonzero tiles, four blocks per SM), the tile walk, the
+    # straddling rows; longer runs: one group walk (after a memset); ebpr:
+    # scan + fix-up; row-balanced: one
     kernels_per_step = 2 if strategy == "ebpr" else 1
+    if strategy == "ebsr" and (knobs.thread_nz << knobs.group_factor) <= 2048:
+        wave = 4 * torch.cuda.get_device_properties(dev).multi_processor_count
+        kernels_per_step = 3 if Ad.nnz > 1024 * wave else 2
 
     def step():
         S.forward(Bd, out=C, workspace=work, stream=stream)

@@ -1,5 +1,5 @@
-// Element-balanced machinery shared by the sequential (ebsr, segment SR) and
-// parallel (ebpr, segment PR) kernels.
+// Element-balanced machinery shared by the group walk (ebsr and segment SR
+// with long chunks) and the parallel kernels (ebpr, segment PR).
 //
 // Work is cut into chunks of consecutive nonzeros.  A row is OWNED by the
 // chunk that holds its first nonzero; the owner writes the row with plain
@@ -8,8 +8,7 @@
 // the last row (continues into the next chunk).  Their FP32 partials go to
 // the chunk's head and tail slots, and each straddling row is assembled
 // once as owner tail + following heads (by the last of its chunks to finish,
-// carry_arrive / seg_carry_arrive, in the ebsr, segment SR and batched
-// walks; by the fix-up kernel, fixup_chunk, after the ebpr and segment PR
+// carry_arrive / seg_carry_arrive, in the group walks; by the fix-up kernel, fixup_chunk, after the ebpr and segment PR
 // kernels) and stored once, so a
 // 16-bit output is rounded once.  Empty rows (empty
 // segments) are written as zero by the chunk holding the next nonzero, so in

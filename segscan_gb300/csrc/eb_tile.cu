@@ -40,7 +40,7 @@ TileGeom tile_geom(int N, int nnz, int dtype, int vmax, bool seg) {
   g.G = std::min(16, ceil_pow2(nv));
   // 17 to 32 wide vectors: one phase of 32 lanes instead of two of 16, unless
   // two full phases gather a matrix's rows as fast (N = 128: 420 against 428
-  // us).  A half empty second phase costs more (N = 100 BF16: ## -> ## us),
+  // us).  A part empty second phase costs more (N = 100 FP32 is 25 vectors),
   // and streamed rows are better read in one piece.
   if (V >= 4 && nv > 16 && nv <= 32 && (seg || nv < 32)) g.G = 32;
   // widths that no wide vector divides: several vectors per lane, as many as

@@ -1,5 +1,7 @@
-// Element-balanced, sequential reduction: ebsr SpMM and the sequential
-// segment_coo family.
+// Element-balanced, sequential reduction by groups with long chunks: ebsr SpMM
+// and the sequential segment_coo family where the caller asks for runs of more
+// than 2048 nonzeros or its scratch holds no tile walk (eb_tile.cuh,
+// seg_tile.cuh: the other calls).
 //
 // Reference counterparts: csrspmm_rowcaching_nnzbalance_cg_kernel
 // (test-cg/include/spmm/spmm_cg.cuh:376-551) and segscan_sr_kernel /

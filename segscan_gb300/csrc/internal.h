@@ -117,7 +117,7 @@ size_t ebsr_walk_workspace(const ss_csr *A, int N, const ss_knobs *knobs);
 // (thread_nz << group_factor) get the group walk with exactly those chunks
 // (less scratch, fewer partial sums); every other tuple gets the tile walk,
 // faster at every width and size measured (1e6 power-law: N = 64 FP32 203
-// against 242 us, N = 4 61 against 110 us, N = 128 BF16 258 against 341 us).
+// against 242 us, N = 4 64 against 112 us, N = 128 BF16 261 against 342 us).
 inline bool tile_tuple(int group_factor, int thread_nz) { return ((long long)thread_nz << group_factor) <= 2048; }
 
 // Launchers (kernels live in spmm_rb.cu, eb_walk.cu, eb_scan.cu).

@@ -1,5 +1,5 @@
-// Device CSR transpose (the backward pass's A^T), value gather and COO ->
-// CSR.
+// Device CSR transpose (the backward pass's A^T), value gather and the entry
+// points of COO -> CSR (sorted in stable_sort.cu).
 //
 // Reference semantics: transpose + compressedRow
 // (test-cg/include/dataloader/dataloader.hpp:109-144), a stable counting

@@ -322,7 +322,7 @@ def extra_precision(A, B, N, fp32_ms, dev):
 
 def extra_batched(dev, N=64, count=512, headline=None):
     """512 CSR matrices (rows log-uniform in [100, 50000], row length Zipf 2.3
-    clipped to [1, 2000], seed 3): one persistent launch replayed from a CUDA
+    clipped to [1, 2000], seed 3): one batched step replayed from a CUDA
     graph (BF16 storage, FP32 accumulation) against one plain FP32 launch per
     matrix, and like for like: batched BF16 against batched FP32 on the same
     matrices, and batched BF16 against the plain FP32 headline SpMM per

@@ -177,9 +177,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 1) fused_bwd_kernel(BwdArgs
       if (kahan) {
         asm volatile("");
         #pragma unroll
-        for (int j = 0; j < NV; j++)
-          #pragma unroll
-          for (int i = 0; i < V; i++) kahan_fma(acc[j][i], comp[j][i], av[u], g[u][j][i]);
+        for (int j = 0; j < NV; j++) kahan_fma<V>(acc[j], comp[j], av[u], g[u][j]);
       } else {
         #pragma unroll
         for (int j = 0; j < NV; j++)

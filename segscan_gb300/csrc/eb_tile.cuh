@@ -111,6 +111,22 @@ __device__ __forceinline__ void store_smem(float *p, const float (&v)[V]) {
   }
 }
 
+template <int V>
+__device__ __forceinline__ void load_smem(const float *p, float (&v)[V]) {
+  if constexpr (V % 4 == 0) {
+    #pragma unroll
+    for (int i = 0; i < V; i += 4) {
+      const float4 x = *reinterpret_cast<const float4 *>(p + i);
+      v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
+    }
+  } else if constexpr (V == 2) {
+    const float2 x = *reinterpret_cast<const float2 *>(p);
+    v[0] = x.x; v[1] = x.y;
+  } else {
+    v[0] = p[0];
+  }
+}
+
 // V elements of the output, widened (plain loads: the row is rewritten here).
 template <typename TC, int V>
 __device__ __forceinline__ void load_old(const TC *p, float (&out)[V]) {
@@ -236,6 +252,35 @@ __device__ __forceinline__ void clear(float (&x)[NV][V]) {
     for (int i = 0; i < V; i++) x[j][i] = 0.f;
 }
 
+// acc = pieces k0 .. k1 - 1 (at(k): V partials in shared memory) added in order
+// with compensation.  A sum that is not finite is added up again without, which
+// gives its Inf or NaN: checking every step instead costs 5 % at N = 4, where
+// the chain of a few pieces is a row's longest (1e6 power-law 63.5 -> 67.2 us).
+template <int V, typename At>
+__device__ __forceinline__ void sum_pieces(int k0, int k1, At at, float (&acc)[V]) {
+  float comp[V], x[V];
+  #pragma unroll
+  for (int i = 0; i < V; i++) acc[i] = comp[i] = 0.f;
+  for (int k = k0; k < k1; k++) {
+    load_smem<V>(at(k), x);
+    #pragma unroll
+    for (int i = 0; i < V; i++) kahan_step(acc[i], comp[i], __fsub_rn(x[i], comp[i]));
+  }
+  bool finite = true;
+  #pragma unroll
+  for (int i = 0; i < V; i++) finite &= fabsf(acc[i]) < INFINITY;
+  if (finite) return;
+  #pragma unroll
+  for (int i = 0; i < V; i++) comp[i] = 0.f;
+  for (int k = k0; k < k1; k++) {
+    load_smem<V>(at(k), x);
+    #pragma unroll
+    for (int i = 0; i < V; i++) comp[i] += x[i];
+  }
+  #pragma unroll
+  for (int i = 0; i < V; i++) acc[i] = fabsf(acc[i]) < INFINITY ? acc[i] : comp[i];
+}
+
 // Row `row` of C = acc (+ the old row in accumulate mode), this lane's columns.
 template <typename TC, int G, int V, int NV, bool ADDC>
 __device__ __forceinline__ void tile_store(const TileProb &p, int N, int row, const float (&acc)[NV][V],
@@ -300,8 +345,7 @@ __device__ __forceinline__ int tile_walk(const TileProb &p, int N, int S, const 
       float b[V];
       unpack_raw<T, V>(raw[u][j], b);
       if (SLOW && kah) {
-        #pragma unroll
-        for (int i = 0; i < V; i++) kahan_fma(acc[j][i], comp[j][i], v, b[i]);
+        kahan_fma<V>(acc[j], comp[j], v, b);
       } else {
         #pragma unroll
         for (int i = 0; i < V; i++) acc[j][i] = fmaf(v, b[i], acc[j][i]);
@@ -542,16 +586,9 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
   auto chain = [&](int s, int x, bool head, float (&acc)[NV][V]) {
     #pragma unroll
     for (int j = 0; j < NV; j++) {
-      float comp[V];
       const int c = lane * V + j * G * V;
-      #pragma unroll
-      for (int i = 0; i < V; i++) acc[j][i] = comp[i] = 0.f;
-      for (int k = max(s, 0); k < x; k++)
-        #pragma unroll
-        for (int i = 0; i < V; i++) kahan_add(acc[j][i], comp[i], s_tail[k * COLS + c + i]);
-      if (head)
-        #pragma unroll
-        for (int i = 0; i < V; i++) kahan_add(acc[j][i], comp[i], s_head[x * COLS + c + i]);
+      sum_pieces<V>(max(s, 0), x + (head ? 1 : 0),
+                    [&](int k) { return (k < x ? s_tail + k * COLS : s_head + x * COLS) + c; }, acc[j]);
     }
   };
   auto to_slot = [&](float *slots, float (&acc)[NV][V]) {

@@ -145,12 +145,14 @@ template <int V, int NV, bool KAHAN>
 __device__ __forceinline__ void add_row(float (&acc)[NV][V], float (&comp)[NV][V], float v,
                                         const float (&b)[NV][V]) {
   #pragma unroll
-  for (int j = 0; j < NV; j++)
-    #pragma unroll
-    for (int i = 0; i < V; i++) {
-      if (KAHAN) kahan_fma(acc[j][i], comp[j][i], v, b[j][i]);
-      else acc[j][i] = fmaf(v, b[j][i], acc[j][i]);
+  for (int j = 0; j < NV; j++) {
+    if (KAHAN) {
+      kahan_fma<V>(acc[j], comp[j], v, b[j]);
+    } else {
+      #pragma unroll
+      for (int i = 0; i < V; i++) acc[j][i] = fmaf(v, b[j][i], acc[j][i]);
     }
+  }
 }
 
 // acc += v * b, compensated when the row is longer than the threshold.

@@ -75,8 +75,7 @@ struct RowWalk {
       float b[V];
       unpack_raw<T, V>(raw[j], b);
       if (kah) {
-        #pragma unroll
-        for (int i = 0; i < V; i++) kahan_fma(acc[j][i], comp[j][i], v, b[i]);
+        kahan_fma<V>(acc[j], comp[j], v, b);
       } else {
         #pragma unroll
         for (int i = 0; i < V; i++) acc[j][i] = fmaf(v, b[i], acc[j][i]);

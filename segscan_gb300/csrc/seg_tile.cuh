@@ -290,22 +290,21 @@ __global__ void __launch_bounds__(TW_T, (ADDC || V * NV > 4 ? 3 : 4)) seg_tile_k
   };
   // a segment's pieces in order: tails of groups [s, x), then the head of x
   auto chain = [&](int s, int x, bool head, float (&acc)[NV][V], int &count) {
-    const float ident = is_max ? -INFINITY : 0.f;
     count = head ? s_hn[x] : 0;
     for (int k = max(s, 0); k < x; k++) count += s_tn[k];
     #pragma unroll
     for (int j = 0; j < NV; j++) {
-      float comp[V];
-      const int c = lane * V + j * G * V;
-      #pragma unroll
-      for (int i = 0; i < V; i++) { acc[j][i] = ident; comp[i] = 0.f; }
-      for (int k = max(s, 0); k < x + (head ? 1 : 0); k++)
+      const int c = lane * V + j * G * V, k0 = max(s, 0), k1 = x + (head ? 1 : 0);
+      auto at = [&](int k) { return (k < x ? s_tail + k * COLS : s_head + x * COLS) + c; };
+      if (is_max) {
         #pragma unroll
-        for (int i = 0; i < V; i++) {
-          const float v = (k < x ? s_tail : s_head)[k * COLS + c + i];
-          if (is_max) acc[j][i] = fmaxf(acc[j][i], v);
-          else kahan_add(acc[j][i], comp[i], v);
-        }
+        for (int i = 0; i < V; i++) acc[j][i] = -INFINITY;
+        for (int k = k0; k < k1; k++)
+          #pragma unroll
+          for (int i = 0; i < V; i++) acc[j][i] = fmaxf(acc[j][i], at(k)[i]);
+      } else {
+        sum_pieces<V>(k0, k1, at, acc[j]);
+      }
     }
   };
   auto to_slot = [&](float *slots, int *counts, float (&acc)[NV][V], int count) {

@@ -137,15 +137,14 @@ __device__ __forceinline__ void rbsr_row(const RbArgs &a, int s, int e, int lane
       #pragma unroll
       for (int u = 0; u < 4; u++)
         #pragma unroll
-        for (int j = 0; j < NV; j++)
-          #pragma unroll
-          for (int i = 0; i < V; i++) {
-            if (KAHAN) {
-              if (q + u < cnt) kahan_fma(acc.v[j][i], comp.v[j][i], v[u], b[u][j][i]);
-            } else {
-              acc.v[j][i] = fmaf(v[u], b[u][j][i], acc.v[j][i]);
-            }
+        for (int j = 0; j < NV; j++) {
+          if (KAHAN) {
+            if (q + u < cnt) kahan_fma<V>(acc.v[j], comp.v[j], v[u], b[u][j]);
+          } else {
+            #pragma unroll
+            for (int i = 0; i < V; i++) acc.v[j][i] = fmaf(v[u], b[u][j][i], acc.v[j][i]);
           }
+        }
     }
   }
 }
@@ -240,15 +239,14 @@ __device__ __forceinline__ void rbpr_slot(const RbArgs &a, int s, int e, int slo
     #pragma unroll
     for (int u = 0; u < U; u++)
       #pragma unroll
-      for (int j = 0; j < NV; j++)
-        #pragma unroll
-        for (int i = 0; i < V; i++) {
-          if (KAHAN) {
-            if (p0 + u * S < e) kahan_fma(acc.v[j][i], comp.v[j][i], v[u], b[u][j][i]);  // not past the row
-          } else {
-            acc.v[j][i] = fmaf(v[u], b[u][j][i], acc.v[j][i]);
-          }
+      for (int j = 0; j < NV; j++) {
+        if (KAHAN) {
+          if (p0 + u * S < e) kahan_fma<V>(acc.v[j], comp.v[j], v[u], b[u][j]);  // not past the row
+        } else {
+          #pragma unroll
+          for (int i = 0; i < V; i++) acc.v[j][i] = fmaf(v[u], b[u][j][i], acc.v[j][i]);
         }
+      }
   }
 }
 

@@ -1,0 +1,70 @@
+"""Infinities in the terms of a sum: a row (or segment) with one is infinite, whatever piece, tile or
+chunk of the walk holds it, one whose partial sums overflow too, and one with both signs is NaN; every
+other row keeps its value (1e-5 of sum|terms|)."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# short rows, rows across pieces and tiles (8 to 128 nonzeros, 128 to 2048), one above the compensation
+# threshold of 1024, one of every length in between
+LENGTHS = [3, 10, 37, 5, 300, 1500, 9, 64, 0, 65, 700, 1, 20, 130, 2]
+SPMM = [("ebsr", {}), ("ebsr", dict(thread_nz=256)), ("rbsr", {}), ("rbpr", {}), ("ebpr", {})]
+KINDS = {"inf": (np.inf, 0.0), "neg": (-np.inf, 0.0), "overflow": (3e38, 3e38), "both": (np.inf, -np.inf)}
+
+
+def placed(n, N, first, kind):
+    """Terms in (0, 1): column j has the kind's values at elements first + j and first + j + 1."""
+    x = np.random.default_rng(5).uniform(0.1, 1, (n, N)).astype(np.float32)
+    rows = np.repeat(np.arange(len(LENGTHS)), LENGTHS)
+    want = np.zeros((len(LENGTHS), N))
+    np.add.at(want, rows, x.astype(np.float64))
+    with np.errstate(invalid="ignore"):
+        for j in range(N):
+            p = min(first + j, n - 2)
+            for q, v in zip((p, p + 1), KINDS[kind]):
+                if v != 0.0:
+                    want[rows[q], j] += v - float(x[q, j])
+                    x[q, j] = v
+        return x, np.where(np.abs(want) > 3.4e38, np.sign(want) * np.inf, want)
+
+
+def check(got, want, what):
+    got = got.double().cpu().numpy()
+    assert np.array_equal(np.isnan(got), np.isnan(want)), f"{what}: NaN"
+    assert np.array_equal(np.isinf(got), np.isinf(want)), f"{what}: Inf"
+    inf = np.isinf(want)
+    assert np.array_equal(np.sign(got[inf]), np.sign(want[inf])), f"{what}: sign"
+    fin = np.isfinite(want)
+    assert np.all(np.abs(got[fin] - want[fin]) <= 1e-5 * np.abs(want[fin])), what
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+@pytest.mark.parametrize("strategy,kw", SPMM)
+@pytest.mark.parametrize("N", [4, 33, 64])
+def test_spmm(cuda, N, strategy, kw, kind):
+    from segscan_gb300 import api
+    n = sum(LENGTHS)
+    indptr = np.concatenate([[0], np.cumsum(LENGTHS)]).astype(np.int32)
+    A = api.CsrMatrix(len(LENGTHS), n, torch.from_numpy(indptr).cuda(), torch.arange(n, dtype=torch.int32, device="cuda"),
+                      torch.ones(n, device="cuda"))
+    for first in list(range(0, 420, max(N, 24))) + list(range(1000, n, 170)):
+        B, want = placed(n, N, first, kind)
+        got = api.spmm(A, torch.from_numpy(B).cuda(), strategy, knobs=api.make_knobs(strategy, N, **kw) if kw else None)
+        check(got, want, f"N={N} first={first}")
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+@pytest.mark.parametrize("reduce", ["sum", "mean"])
+@pytest.mark.parametrize("strategy", ["sr", "pr"])
+@pytest.mark.parametrize("N", [4, 33, 64])
+def test_segment(cuda, N, strategy, reduce, kind):
+    from segscan_gb300 import api
+    n, M = sum(LENGTHS), len(LENGTHS)
+    index = torch.from_numpy(np.repeat(np.arange(M), LENGTHS).astype(np.int32)).cuda()
+    for first in list(range(0, 420, max(N, 24))) + list(range(1000, n, 170)):
+        x, want = placed(n, N, first, kind)
+        if reduce == "mean":
+            want = want / np.maximum(LENGTHS, 1)[:, None]
+        check(api.segment(torch.from_numpy(x).cuda(), index, M, reduce, strategy), want, f"N={N} first={first}")

@@ -414,18 +414,19 @@ size_t bucket_smem(int F) { return (size_t)(F + 2 + 2 * CHUNK2 + (T2 / 32) * ((F
 }  // namespace
 
 StableSortPlan stable_sort_plan(int K, int nnz) {
-  StableSortPlan p;
+  StableSortPlan p{};
+  if (K <= 0 || nnz <= 0) return p;  // nothing to sort (and no ranges to divide the elements by)
   // buckets of at most 6144 elements on average (a chunk holds 8192), more
   // keys per bucket where there would be too many buckets
   int f = F_LOG2_MAX;
-  const double avg = K > 0 ? (double)nnz / K : 0.0;
+  const double avg = (double)nnz / K;
   while (f > 0 && (double)(1 << f) * avg > 6144.0) f--;
   long long nb = ((long long)K + (1LL << f) - 1) >> f;
   while (nb > NB_MAX && f < F_LOG2_MAX) {
     f++;
     nb = ((long long)K + (1LL << f) - 1) >> f;
   }
-  p.ok = K > 0 && nnz > 0 && nb <= NB_MAX;
+  p.ok = nb <= NB_MAX;
   p.f = f;
   p.NB = (int)nb;
   // level 1: one range per resident block (two per SM while both blocks' count

@@ -207,3 +207,11 @@ def test_python_api_refuses_host_tensors_and_bad_shapes(lib):
         api.default_knobs("csr_magic", 4)
     with pytest.raises(TypeError, match="unknown knob"):
         api.make_knobs("ebsr", 4, warp_count=2)
+
+
+@pytest.mark.parametrize("nrow", [0, 1, 5, 5000, 20_000_000])
+def test_coo_workspace_of_an_empty_edge_list(lib, nrow):
+    """No edges: a size of a few bytes, and no division by the (zero) edges a block owns."""
+    n = ctypes.c_size_t()
+    assert lib.ss_coo_to_csr_workspace_size(nrow, 0, ctypes.byref(n)) == 0
+    assert n.value > 0

@@ -24,6 +24,29 @@ struct NvtxRange {
 ss_status fail(ss_status st, const char *fmt, ...);
 ss_status cuda_fail(cudaError_t err, const char *what);
 
+// Lets the kernel take up to `most` bytes of dynamic shared memory.  The limit
+// belongs to the kernel, not to the calling thread: `most` is the largest that
+// any call of this kernel takes, whatever the sizes of this one, so that no
+// thread lowers the limit between another's call and its launch.
+inline ss_status allow_smem(const void *fn, size_t most, const char *what) {
+  if (most <= 48 * 1024) return SS_OK;  // allowed anyway
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  return e == cudaSuccess ? SS_OK : cuda_fail(e, what);
+}
+
+// One launch, checked, so that no kernel runs on what a refused one before it
+// did not write.
+template <typename... P, typename... A>
+ss_status launch(const char *what, void (*fn)(P...), long long blocks, int threads, size_t smem, cudaStream_t s,
+                 const A &...a) {
+  auto go = [&](P... p) {
+    void *args[] = {(void *)&p...};
+    return cudaLaunchKernel((const void *)fn, dim3((unsigned)blocks), dim3((unsigned)threads), args, smem, s);
+  };
+  cudaError_t e = go(a...);
+  return e == cudaSuccess ? SS_OK : cuda_fail(e, what);
+}
+
 // One SpMM problem after argument checks.
 struct SpmmCall {
   int M, K, N, nnz;

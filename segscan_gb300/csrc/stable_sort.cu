@@ -451,20 +451,15 @@ ss_status stable_sort(const StableSortPlan &p, SortArgs &a, void *ws, cudaStream
   a.rec = (int2 *)w; w += align256((size_t)a.nnz * 8);
   a.rkey = (int32_t *)w;
   a.f = p.f; a.F = 1 << p.f; a.nb_bits = ilog2(p.NB); a.NB = p.NB; a.ranges = p.ranges; a.range = p.range;
-  const size_t psm = partition_smem(p.NB);
-  const size_t bsm = bucket_smem(a.F);
-  cudaError_t e = cudaFuncSetAttribute(partition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(bucket_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm);
-  if (e != cudaSuccess) return cuda_fail(e, "stable sort attributes");
-  range_count_kernel<<<p.ranges, 1024, (size_t)p.NB * 4, s>>>(a);
-  range_prefix_kernel<<<ceil_div(p.NB, 8), 256, 0, s>>>(a);
-  partition_kernel<<<p.ranges, PT, psm, s>>>(a);
+  ss_status st = allow_smem((const void *)partition_kernel, partition_smem(NB_MAX), "stable sort partition");
+  if (st == SS_OK) st = allow_smem((const void *)bucket_kernel, bucket_smem(1 << F_LOG2_MAX), "stable sort buckets");
+  if (st == SS_OK) st = launch("stable sort counts", range_count_kernel, p.ranges, 1024, (size_t)p.NB * 4, s, a);
+  if (st == SS_OK) st = launch("stable sort prefix", range_prefix_kernel, ceil_div(p.NB, 8), 256, 0, s, a);
+  if (st == SS_OK) st = launch("stable sort partition", partition_kernel, p.ranges, PT, partition_smem(p.NB), s, a);
+  if (st != SS_OK) return st;
   if (p.f == 0)
-    single_key_kernel<<<std::min(ceil_div(a.nnz, 256), sm_count() * 8), 256, 0, s>>>(a);
-  else
-    bucket_kernel<<<p.NB, T2, bsm, s>>>(a);
-  e = cudaGetLastError();
-  return e == cudaSuccess ? SS_OK : cuda_fail(e, "stable sort launch");
+    return launch("stable sort", single_key_kernel, std::min(ceil_div(a.nnz, 256), sm_count() * 8), 256, 0, s, a);
+  return launch("stable sort buckets", bucket_kernel, p.NB, T2, bucket_smem(a.F), s, a);
 }
 
 }  // namespace ss

@@ -1,0 +1,86 @@
+"""A kernel's shared memory limit is one number for all host threads: a call that set it to its own size
+could lower it between another thread's set and launch.  So every call sets the same value, at least what
+any launch takes (above the default 48 KB).  The library's host code runs here against recorded CUDA calls."""
+import concurrent.futures as cf
+import ctypes
+import subprocess
+from pathlib import Path
+
+import pytest
+
+from segscan_gb300 import build
+from segscan_gb300._lib import SsCsr, SsKnobs
+
+HERE = Path(__file__).resolve().parent
+PTR = 1 << 20  # device pointers are never dereferenced on the host
+
+
+@pytest.fixture(scope="module")
+def rec(lib, tmp_path_factory):
+    out = tmp_path_factory.mktemp("recorded")
+    srcs = [s for s in sorted(build.CSRC.glob("*.cu"))
+            if s.stem in ("util", "backward", "sddmm") or "smem" in s.read_text()]
+
+    def compile(src):
+        obj = out / (src.stem + ".o")
+        subprocess.run([build.nvcc(), *build.ARCH, "-std=c++17", "-O0", "-Xcicc", "-O0", "-Xptxas", "-O0", "-Xcompiler",
+                        "-fPIC", "--expt-relaxed-constexpr", "-include", str(HERE / "cpp" / "record_launches.h"), "-I",
+                        str(build.INCLUDE), "-c", str(src), "-o", str(obj)], check=True)
+        return obj
+
+    with cf.ThreadPoolExecutor(8) as ex:
+        objs = list(ex.map(compile, srcs))
+    rest = [build.BUILD / (s.stem + ".o") for s in sorted(build.CSRC.glob("*.cu")) if s not in srcs]
+    so = out / "librecorded.so"
+    subprocess.run([build.nvcc(), *build.ARCH, "-shared", "-o", str(so), *map(str, objs + rest)], check=True)
+    return ctypes.CDLL(str(so))
+
+
+def calls(rec, run):
+    """[(kernel, bytes, is a launch)] of the CUDA calls that run() makes."""
+    lo = rec.recorded_count()
+    run()
+    out = []
+    for i in range(lo, rec.recorded_count()):
+        fn, n, launch = ctypes.c_void_p(), ctypes.c_longlong(), ctypes.c_int()
+        rec.recorded_get(ctypes.c_longlong(i), ctypes.byref(fn), ctypes.byref(n), ctypes.byref(launch))
+        out.append((fn.value, n.value, bool(launch.value)))
+    return out
+
+
+def check(seen):
+    """One limit per kernel, above all its launches; returns how many kernels set one."""
+    limits, launches = {}, {}
+    for fn, n, launch in seen:
+        (launches if launch else limits).setdefault(fn, set()).add(n)
+    for fn, values in limits.items():
+        assert len(values) == 1, f"limits {sorted(values)}"
+        assert max(values) <= 227 * 1024
+        assert max(launches.get(fn, {0})) <= max(values), "launched above its limit"
+    for fn, sizes in launches.items():
+        assert fn in limits or max(sizes) <= 48 * 1024, f"{max(sizes)} bytes without a limit"
+    return len(limits)
+
+
+def ok(status, rec):
+    rec.ss_last_error.restype = ctypes.c_char_p
+    assert status == 0, rec.ss_last_error()
+
+
+def big(n=1 << 40):
+    return ctypes.c_size_t(n)
+
+
+SIZES = [(1000, 5000), (4000, 60_000), (60_000, 200_000), (300_000, 1_000_000), (1_000_000, 4_600_000),
+         (2_000_000, 4_000_000), (16_000_000, 20_000_000)]
+
+
+def test_coo_to_csr(rec):
+    def run():
+        for nrow, nnz in SIZES:
+            ok(rec.ss_coo_to_csr_values(nrow, nnz, ctypes.c_void_p(PTR), ctypes.c_void_p(PTR), ctypes.c_void_p(PTR), 0,
+                                        *[ctypes.c_void_p(PTR)] * 5, big(), None), rec)
+
+    seen = calls(rec, run)
+    assert check(seen) == 2
+    assert sum(launch for _, _, launch in seen) == 4 * len(SIZES)

@@ -417,14 +417,12 @@ ss_status launch_rbsr(const SpmmCall &c, const RbGeom &geom, cudaStream_t s) {
   const int most = addc ? 768 : 1024;
   const int threads = (int)std::min((long long)most, (per * g.G + 31) / 32 * 32);
   const int NG = threads / g.G;
-  const size_t smem = (size_t)3 * NG * (ROW_CAP + 4) * 4;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_fail(e, "rbsr shared memory");
-  }
+  const size_t group_smem = (size_t)3 * (ROW_CAP + 4) * 4;
+  const ss_status st = allow_smem(fn, group_smem * (most / g.G), "rbsr shared memory");
+  if (st) return st;
   void *args[] = {&a};
   cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)ceil_div(c.M, a.block_rows), (unsigned)g.phases, 1),
-                                   dim3(threads, 1, 1), args, smem, s);
+                                   dim3(threads, 1, 1), args, group_smem * NG, s);
   return e == cudaSuccess ? SS_OK : cuda_fail(e, "rbsr launch");
 }
 ss_status launch_rbpr(const SpmmCall &c, const RbGeom &g, cudaStream_t s) { return launch_rb(true, c, g, s); }

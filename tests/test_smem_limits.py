@@ -84,3 +84,22 @@ def test_coo_to_csr(rec):
     seen = calls(rec, run)
     assert check(seen) == 2
     assert sum(launch for _, _, launch in seen) == 4 * len(SIZES)
+
+
+def spmm_calls(rec, strategy, **knobs):
+    n = ctypes.c_size_t()
+    for nrow, nnz in [(100, 700)] + SIZES[:6]:
+        for N in (1, 4, 8, 32, 47, 64, 100, 128, 300):
+            for dtype in (0, 1):
+                for accumulate in (0, 1):
+                    A = SsCsr(nrow, nrow, nnz, PTR, PTR, PTR, dtype)
+                    k = SsKnobs()
+                    ok(rec.ss_default_knobs(strategy, N, ctypes.byref(k)), rec)
+                    for name, v in knobs.items():
+                        setattr(k, name, v)
+                    ok(rec.ss_spmm(strategy, ctypes.byref(A), N, ctypes.c_void_p(PTR), ctypes.c_void_p(PTR), 0,
+                                   accumulate, ctypes.byref(k), ctypes.c_void_p(PTR), big(), None), rec)
+
+
+def test_rbsr(rec):
+    assert check(calls(rec, lambda: spmm_calls(rec, 3))) >= 4

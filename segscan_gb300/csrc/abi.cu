@@ -194,7 +194,7 @@ ss_status geom_sr(long long worker_units, int nnz, int N, int dtype, int val_byt
   while (stage > 8 && sr_smem_bytes(stage, g.workers_per_block, val_bytes) > 48 * 1024) stage >>= 1;
   g.stage = stage;
   g.smem = sr_smem_bytes(stage, g.workers_per_block, val_bytes);
-  if (g.smem > 200 * 1024)
+  if (g.smem > SR_SMEM_MAX)
     return fail(SS_ERR_UNSUPPORTED_KNOBS, "%d groups per block need %zu B of shared memory",
                 g.workers_per_block, g.smem);
   // reference grid: worker_units * block_factor blocks of thread_per_block

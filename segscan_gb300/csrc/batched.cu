@@ -293,8 +293,8 @@ ss_status ss_spmm_batched(const void *host_plan, void *dev_plan, void *stream) {
   else fn = batched_kernel_f16(h.V, h.NV, h.c_dtype == SS_F32);
   if (!fn) return fail(SS_ERR_UNSUPPORTED_KNOBS, "no batched kernel for V=%d NV=%d", h.V, h.NV);
   if (h.smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.smem);
-    if (e != cudaSuccess) return cuda_fail(e, "batched smem attribute");
+    const ss_status st = allow_smem(fn, SR_SMEM_MAX, "batched smem attribute");
+    if (st) return st;
   }
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, h.block, h.smem);

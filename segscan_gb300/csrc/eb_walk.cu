@@ -33,8 +33,8 @@ size_t sr_smem_bytes(int stage, int workers_per_block, int val_bytes) {
 static ss_status run_sr(void *fn, void *arg, const EbGeom &g, size_t smem, cudaStream_t s, const char *what) {
   if (!fn) return fail(SS_ERR_UNSUPPORTED_KNOBS, "no %s kernel for V=%d NV=%d", what, g.cs.V, g.cs.NV);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_fail(e, what);
+    const ss_status st = allow_smem(fn, SR_SMEM_MAX, what);
+    if (st) return st;
   }
   // at most one resident wave; workers stride over the chunks
   int per_sm = 0;

@@ -117,6 +117,7 @@ size_t seg_sr_workspace_bytes(const EbGeom &g, int N);
 ss_status geom_sr(long long worker_units, int nnz, int N, int dtype, int val_bytes, const ss_knobs &k, EbGeom &g);
 // shared memory of the sequential-walk kernels (eb_walk.cu)
 size_t sr_smem_bytes(int stage, int workers_per_block, int val_bytes);
+constexpr size_t SR_SMEM_MAX = 200 * 1024;  // the most a tuple may ask for
 // device address of the bounded-wait status word (eb_walk.cu)
 int *walk_error_ptr();
 // streaming multiprocessors of the current device, looked up once per device

@@ -103,3 +103,57 @@ def spmm_calls(rec, strategy, **knobs):
 
 def test_rbsr(rec):
     assert check(calls(rec, lambda: spmm_calls(rec, 3))) >= 4
+
+
+@pytest.mark.parametrize("thread_nz", [2, 256])
+def test_ebsr_tile_and_group_walk(rec, thread_nz):
+    def run():
+        for block in (64, 256, 512):
+            for gf in (0, 2, 4, 5):
+                tnz = thread_nz if thread_nz < 256 else 4096 >> gf
+                spmm_calls(rec, 2, thread_nz=tnz, group_factor=gf, thread_per_block=block)
+
+    assert check(calls(rec, run)) > 0
+
+
+def test_segment(rec):
+    def run():
+        for n in (100, 5000, 60_000, 1_000_000, 4_600_000):
+            for N in (1, 4, 8, 47, 64, 128):
+                for dtype in (0, 1):
+                    for accumulate in (0, 1):
+                        for gf, tnz in ((0, 1), (2, 8), (4, 8), (4, 256), (0, 4096)):
+                            k = SsKnobs()
+                            ok(rec.ss_default_knobs(2, N, ctypes.byref(k)), rec)
+                            k.group_factor, k.thread_nz = gf, tnz
+                            ok(rec.ss_segment_coo(1, ctypes.c_void_p(PTR), dtype, ctypes.c_void_p(PTR), n, N, n,
+                                                  ctypes.c_void_p(PTR), 0, accumulate, ctypes.byref(k),
+                                                  ctypes.c_void_p(PTR), big(), None), rec)
+
+    check(calls(rec, run))
+
+
+def test_batched(rec):
+    def run():
+        for sizes in ([(50, 100)] * 3, [(3000, 40_000)] * 40, [(50_000, 300_000)] * 60):
+            for N in (1, 4, 8, 32, 64, 128):
+                for dtype in (0, 1):
+                    for block in (64, 256, 512):
+                        for gf, tnz in ((0, 4), (4, 8), (5, 256), (0, 4096)):
+                            count = len(sizes)
+                            mats = (SsCsr * count)(*[SsCsr(m, m, n, PTR, PTR, PTR, dtype) for m, n in sizes])
+                            knobs = (SsKnobs * count)()
+                            for k in knobs:
+                                ok(rec.ss_default_knobs(2, N, ctypes.byref(k)), rec)
+                                k.group_factor, k.thread_nz, k.thread_per_block = gf, tnz, block
+                            kinds = (ctypes.c_int * count)(*[2 if i % 3 else 3 for i in range(count)])
+                            ptrs = (ctypes.c_void_p * count)(*[PTR] * count)
+                            host, dev = ctypes.c_size_t(), ctypes.c_size_t()
+                            ok(rec.ss_batch_plan_size_ex(count, mats, N, knobs, kinds, ctypes.byref(host),
+                                                         ctypes.byref(dev)), rec)
+                            plan = ctypes.create_string_buffer(host.value)
+                            ok(rec.ss_batch_plan_ex(count, mats, N, ptrs, ptrs, 0, knobs, kinds, plan, host,
+                                                    ctypes.c_void_p(PTR), dev, None), rec)
+                            ok(rec.ss_spmm_batched(plan, ctypes.c_void_p(PTR), None), rec)
+
+    assert check(calls(rec, run)) > 0

@@ -377,6 +377,9 @@ struct BucketPlan {
 static int sort_bytes(int F, int cap) { return (4 + 3 * (cap + 8) + 2 * cap + 2 * F + 1 + 64) * 4; }
 static int sort_cap(int F) { return ((TB_SORT_SMEM - sort_bytes(F, 0)) / 20) & ~3; }
 
+// Shared memory of a partition block: three words per bucket, the staged tile.
+static size_t part_bytes(int NB) { return (size_t)(3 * NB + 1 + 3 * TB_E) * 4; }
+
 static BucketPlan bucket_plan(int K, int nnz) {
   BucketPlan p;
   const double avg = K > 0 ? (double)nnz / K : 0.0;
@@ -935,24 +938,24 @@ static ss_status bucket_transpose(const ss_csr *A, const BucketPlan &pl, int32_t
   const int sms = sm_count();
   cudaError_t e = cudaMemsetAsync(w.count, 0, (size_t)pl.NB * 4, s);
   if (e != cudaSuccess) return cuda_fail(e, "transpose clear");
-  const size_t hist_smem = (size_t)pl.NB * 4;
-  const size_t part_smem = (size_t)(3 * pl.NB + 1 + 3 * TB_E) * 4;
-  const size_t sort_smem = (size_t)sort_bytes(pl.F, pl.cap);
-  e = cudaFuncSetAttribute(bucket_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(bucket_partition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part_smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(bucket_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem);
-  if (e != cudaSuccess) return cuda_fail(e, "transpose attributes");
+  ss_status st = allow_smem((const void *)bucket_partition_kernel, part_bytes(TB_NB_MAX), "transpose partition");
+  if (st == SS_OK) st = allow_smem((const void *)bucket_sort_kernel, TB_SORT_SMEM, "transpose sort");
+  if (st != SS_OK) return st;
   const long long tiles = ((long long)nnz + TB_E - 1) / TB_E;
-  const int count_blocks = (int)std::min<long long>(((long long)nnz + 4 * TB_T - 1) / (4 * TB_T), 2LL * sms);
-  bucket_count_kernel<<<count_blocks, TB_T, hist_smem, s>>>(A->indices, nnz, K, pl.f, pl.NB, w.count);
-  bucket_scan_kernel<<<1, TB_T, 0, s>>>(w.count, pl.NB, nnz, K, w.start, w.cursor, t_indptr, perm, t_indices);
+  const long long count_blocks = std::min<long long>(((long long)nnz + 4 * TB_T - 1) / (4 * TB_T), 2LL * sms);
+  st = launch("transpose counts", bucket_count_kernel, count_blocks, TB_T, (size_t)pl.NB * 4, s, A->indices, nnz, K,
+              pl.f, pl.NB, w.count);
+  if (st == SS_OK)
+    st = launch("transpose scan", bucket_scan_kernel, 1, TB_T, 0, s, w.count, pl.NB, nnz, K, w.start, w.cursor, t_indptr,
+                perm, t_indices);
   PartArgs pa;
   pa.indptr = A->indptr; pa.cols = A->indices;
   pa.M = M; pa.K = K; pa.nnz = nnz; pa.f = pl.f; pa.NB = pl.NB;
   pa.cursor = w.cursor; pa.pos = w.pos; pa.row = w.row; pa.col = w.col;
-  bucket_partition_kernel<<<(int)std::min<long long>(tiles, (long long)sms * TB_PART_BLOCKS), TB_PT, part_smem, s>>>(pa);
+  if (st == SS_OK)
+    st = launch("transpose partition", bucket_partition_kernel, std::min<long long>(tiles, (long long)sms * TB_PART_BLOCKS),
+                TB_PT, part_bytes(pl.NB), s, pa);
+  if (st != SS_OK) return st;
   BucketSortArgs sa;
   sa.start = w.start; sa.pos = w.pos; sa.row = w.row; sa.col = w.col;
   sa.K = K; sa.NB = pl.NB; sa.f = pl.f; sa.F = pl.F; sa.cap = pl.cap;
@@ -961,9 +964,8 @@ static ss_status bucket_transpose(const ss_csr *A, const BucketPlan &pl, int32_t
   sa.t_vals = t_vals;
   sa.vsize = dtype_size(A->value_dtype);
   sa.err = walk_error_ptr();
-  bucket_sort_kernel<<<std::min(pl.NB, sms * TB_SORT_BLOCKS), TB_ST, sort_smem, s>>>(sa);
-  e = cudaGetLastError();
-  return e == cudaSuccess ? SS_OK : cuda_fail(e, "transpose launch");
+  return launch("transpose sort", bucket_sort_kernel, std::min(pl.NB, sms * TB_SORT_BLOCKS), TB_ST,
+                (size_t)sort_bytes(pl.F, pl.cap), s, sa);
 }
 
 }  // namespace ss

@@ -157,3 +157,15 @@ def test_batched(rec):
                             ok(rec.ss_spmm_batched(plan, ctypes.c_void_p(PTR), None), rec)
 
     assert check(calls(rec, run)) > 0
+
+
+def test_transpose(rec):
+    def run():
+        for n, nnz in [(10, 5)] + SIZES:
+            A = SsCsr(n, n, nnz, PTR, PTR, PTR, 0)
+            ok(rec.ss_csr_transpose(ctypes.byref(A), *[ctypes.c_void_p(PTR)] * 4, big(), None),
+               rec)
+
+    seen = calls(rec, run)
+    assert check(seen) == 2
+    assert sum(launch for _, _, launch in seen) == 4 * (len(SIZES) + 1)

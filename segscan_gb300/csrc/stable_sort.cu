@@ -199,6 +199,8 @@ __global__ void __launch_bounds__(PT, 2) partition_kernel(SortArgs a) {
     for (long long q = (long long)total + tid; q < a.nnz; q += PT) {  // elements with keys outside [0, K)
       a.perm[q] = -1;
       a.out_payload[q] = -1;
+      if (a.out_vals && a.vsize == 4) ((uint32_t *)a.out_vals)[q] = 0u;
+      else if (a.out_vals) ((uint16_t *)a.out_vals)[q] = 0;
     }
   }
   if (blockIdx.x == 0) {

@@ -30,7 +30,7 @@ struct SortArgs {
 StableSortPlan stable_sort_plan(int K, int nnz);
 size_t stable_sort_ws(const StableSortPlan &p, int nnz);
 // perm = positions grouped by key in [0, K), in input order inside a key;
-// elements with other keys land past out_indptr[K] as -1.
+// elements with other keys land past out_indptr[K] as -1, their values as 0.
 ss_status stable_sort(const StableSortPlan &p, SortArgs &a, void *ws, cudaStream_t s);
 
 }  // namespace ss

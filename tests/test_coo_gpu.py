@@ -99,3 +99,18 @@ def test_old_workspace_is_still_accepted(cuda):
     torch.cuda.synchronize()
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("nrow,nnz", [(300, 5000), (6000, 90000), (5, 40000)])
+def test_values_of_rows_outside_are_zero(cuda, nrow, nnz, dtype):
+    """Past indptr[nrow]: -1 in the columns and the permutation, zero in the values, as the one-level sort leaves them."""
+    from segscan_gb300 import api
+    rng = np.random.default_rng(4)
+    rows = rng.integers(-2, nrow + 2, size=nnz).astype(np.int32)
+    A, perm = api.coo_to_csr(nrow, torch.from_numpy(rows).cuda(), torch.zeros(nnz, dtype=torch.int32, device="cuda"),
+                             ncol=1, values=torch.ones(nnz, device="cuda", dtype=dtype))
+    m = int(((rows >= 0) & (rows < nrow)).sum())
+    assert m < nnz and int(A.indptr[-1]) == m
+    assert torch.all(A.values[:m] == 1) and torch.all(A.values[m:] == 0)
+    assert torch.all(A.indices[m:] == -1) and torch.all(perm[m:] == -1)

@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(ADDC ? 768 : 1024, 1) rb_tile_kernel(RowArgs a
         const int i = k * G + lane;
         if ((unsigned)c[k] >= (unsigned)a.K) {
           c[k] = -1;
+          v[k] = 0.f;  // (Inf and NaN times the zero row would not vanish)
           bad = true;
         }
         s_col[i] = c[k];

@@ -68,3 +68,21 @@ def test_segment(cuda, N, strategy, reduce, kind):
         if reduce == "mean":
             want = want / np.maximum(LENGTHS, 1)[:, None]
         check(api.segment(torch.from_numpy(x).cuda(), index, M, reduce, strategy), want, f"N={N} first={first}")
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_rbsr_leaves_out_the_value_of_a_column_outside(cuda, value):
+    """A nonzero whose column is not in the matrix adds nothing, whatever its value."""
+    from segscan_gb300 import api
+    lengths = [3, 10, 70, 5, 1500]
+    n = sum(lengths)
+    indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)).cuda()
+    cols = torch.arange(n, dtype=torch.int32, device="cuda")
+    vals = torch.ones(n, device="cuda")
+    for N in (4, 33, 64):
+        B = torch.rand(n, N, device="cuda")
+        ref = api.spmm(api.CsrMatrix(len(lengths), n, indptr, cols, vals.index_fill(0, cols[::9].long(), 0)), B, "rbsr")
+        bad, v = cols.clone(), vals.clone()
+        bad[::18], bad[9::18], v[::9] = n, -1, value
+        got = api.spmm(api.CsrMatrix(len(lengths), n, indptr, bad, v), B, "rbsr")
+        assert torch.all((got - ref).abs() <= 1e-5 * ref.abs()), f"N={N}"

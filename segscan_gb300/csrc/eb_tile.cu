@@ -7,7 +7,8 @@
 namespace ss {
 
 // row_start[t] = first row that starts at or after nonzero t * tile_nz
-// (row_start[tiles] = M), four rows a thread.  2 us on a million rows, against
+// (row_start[tiles] = M; also M where indptr[M] ends before the tile does, as
+// in matrices whose dropped entries follow the last row), four rows a thread.  2 us on a million rows, against
 // 2.5 us of search latency in every wave of the walk (N = 64: 207 -> 203 us).
 __global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restrict__ indptr, int M, int tile,
                                                         uint32_t inv_tile, int tiles, int32_t *__restrict__ row_start) {
@@ -22,7 +23,8 @@ __global__ void __launch_bounds__(256) tile_rows_kernel(const int32_t *__restric
     int x[5];
     x[0] = r0 > 0 ? tile_of(__ldg(indptr + r0 - 1)) : -1;
     #pragma unroll
-    for (int i = 0; i < 4; i++) x[i + 1] = r0 + i <= M ? tile_of(__ldg(indptr + r0 + i)) : INT_MIN;
+    for (int i = 0; i < 4; i++)
+      x[i + 1] = r0 + i < M ? tile_of(__ldg(indptr + r0 + i)) : r0 + i == M ? tiles : INT_MIN;
     #pragma unroll
     for (int i = 0; i < 4; i++)
       for (int t = max(x[i] + 1, 0); t <= min(x[i + 1], tiles - 1); t++) row_start[t] = (int)r0 + i;

@@ -1,0 +1,66 @@
+"""Matrices whose arrays go on after the last row (indptr[nrow] < nnz, columns -1): COO -> CSR makes them of
+edges with rows outside the matrix, the transpose of columns outside it.  Every row of C is written and
+right, above and below one wave of tiles, whatever the scratch held before (1e-5 of sum|a*b|)."""
+import numpy as np
+import pytest
+import torch
+
+import oracle_lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(params=[0, 1, 255])
+def scratch(request, monkeypatch):
+    from segscan_gb300 import api
+    monkeypatch.setattr(api, "_workspace",
+                        lambda n, device: torch.full((n + 256,), request.param, dtype=torch.uint8, device=device))
+    return request.param
+
+
+def dropping(nnz, nrow, dropped, seed=2):
+    """rows, cols (int32) with `dropped` rows outside, the last 40 rows of the matrix and some others empty."""
+    rng = np.random.default_rng(seed)
+    rows = rng.integers(0, nrow - 40, size=nnz)
+    rows[rows % 5 == 2] += 1
+    rows[rng.permutation(nnz)[:dropped]] = nrow + 3
+    return rows.astype(np.int32), rng.integers(0, nrow, size=nnz).astype(np.int32)
+
+
+def expect(rows, cols, vals, nrow, B):
+    keep = np.flatnonzero(rows < nrow)
+    order = keep[np.argsort(rows[keep], kind="stable")]
+    indptr = np.concatenate([[0], np.cumsum(np.bincount(rows[keep], minlength=nrow))]).astype(np.int32)
+    return oracle_lib.spmm_f64(indptr, cols[order], vals[order], B, threads=8)
+
+
+@pytest.mark.parametrize("N,nnz", [(4, 9000), (4, 1_500_000), (64, 9000), (64, 900_000), (33, 900_000)])
+@pytest.mark.parametrize("dropped", [1, 700, 6000])
+def test_spmm(cuda, scratch, N, nnz, dropped):
+    from segscan_gb300 import api
+    nrow = 5000
+    rows, cols = dropping(nnz, nrow, dropped)
+    vals = np.random.default_rng(1).uniform(-1, 1, nnz).astype(np.float32)
+    A, _ = api.coo_to_csr(nrow, torch.from_numpy(rows).cuda(), torch.from_numpy(cols).cuda(), ncol=nrow,
+                          values=torch.from_numpy(vals).cuda())
+    B = np.random.default_rng(7).uniform(-1, 1, (nrow, N)).astype(np.float32)
+    got = api.spmm(A, torch.from_numpy(B).cuda(), "ebsr").double().cpu().numpy()
+    want, terms = expect(rows, cols, vals, nrow, B)
+    assert np.all(np.abs(got - want) <= 1e-5 * terms + 1e-30)
+
+
+@pytest.mark.parametrize("N", [4, 64])
+def test_gradient_of_B(cuda, scratch, N):
+    """dB = A^T dC where A has columns outside: A^T's arrays go on after its last row."""
+    from segscan_gb300 import api, autograd
+    nnz, n = 1_500_000, 5000
+    cols, rows = dropping(nnz, n, 6000)
+    rows = np.sort(rows)
+    indptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int32)
+    vals = np.random.default_rng(1).uniform(-1, 1, nnz).astype(np.float32)
+    A = api.CsrMatrix(n, n, torch.from_numpy(indptr).cuda(), torch.from_numpy(cols).cuda(), torch.from_numpy(vals).cuda())
+    B = torch.zeros(n, N, device="cuda", requires_grad=True)
+    dC = np.random.default_rng(7).uniform(-1, 1, (n, N)).astype(np.float32)
+    autograd.spmm(A, A.values, B).backward(torch.from_numpy(dC).cuda())
+    want, terms = expect(cols, rows, vals, n, dC)
+    assert np.all(np.abs(B.grad.double().cpu().numpy() - want) <= 1e-5 * terms + 1e-30)

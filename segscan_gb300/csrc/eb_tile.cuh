@@ -319,7 +319,8 @@ __device__ __forceinline__ int tile_walk(const TileProb &p, int N, int S, const 
   for (int j = 0; j < NV; j++) {
     // a lane past the last column repeats a column that it (or lane 0)
     // computes too and stores the same value to the same place: no predicate
-    // per load and store
+    // per load and store (accumulating, such lanes leave the walk to the
+    // others: they could read a row after another lane's store)
     const int cj = act[j] ? col0 + j * G * V : act[0] ? col0 : col0 - lane * V;
     Bj[j] = (const char *)((const T *)p.B + cj);
     Cj[j] = (char *)((TC *)p.C + cj) - ldc;  // marks hold row + 1
@@ -432,7 +433,6 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
   const int tile = item - p.item_begin;
   const uint64_t keep = policy_keep(a.keep_frac), strm = policy_stream();
   const int lane = tid & (G - 1), g = tid / G;
-  const unsigned mask = G >= 32 ? 0xffffffffu : (((1u << (G & 31)) - 1u) << (wl & ~(G - 1)));
   const int col0 = phase * COLS + lane * V;
   bool act[NV];
   #pragma unroll
@@ -567,7 +567,9 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
   // accumulating into 16 bits is rare: one instantiation, the one that fits all
   constexpr bool FAST = !(ADDC && sizeof(TC) == 2);
   int hr;
-  if (FAST && !slow)
+  if (ADDC && !act[0])
+    hr = 0;
+  else if (FAST && !slow)
     hr = tile_walk<T, TC, G, V, NV, !FAST, ADDC>(p, a.N, S, s_col + gb, s_val + gb, s_info + gb, s_kb, g * S, shead,
                                            stail, lane, col0, act, keep, strm);
   else

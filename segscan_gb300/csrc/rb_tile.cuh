@@ -51,6 +51,8 @@ struct RowWalk {
     #pragma unroll
     for (int j = 0; j < NV; j++) {
       // lanes past the last column repeat one that this lane (or lane 0) has
+      // (accumulating, they leave the walk to the others: they could read a
+      // row after another lane's store)
       const int cj = act[j] ? col0 + j * G * V : act[0] ? col0 : col0 - lane * V;
       Bj[j] = (const char *)((const T *)a.B + cj);
       Cj[j] = (char *)((TC *)a.C + cj) - ldc;
@@ -190,6 +192,7 @@ __global__ void __launch_bounds__(ADDC ? 768 : 1024, 1) rb_tile_kernel(RowArgs a
       if (re > rs && pos < (unsigned)n) s_info[pos] = r0 + lane + 1;
       bad = __any_sync(mask, bad);
       __syncwarp(mask);  // the marks are visible to the group
+      if (ADDC && !act[0]) continue;
       if (!bad) {
         at_start = true;  // for a later chunk: look the row up
         int q = 0;

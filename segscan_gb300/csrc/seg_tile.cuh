@@ -88,6 +88,7 @@ __device__ __forceinline__ int seg_walk(const SegTileArgs &a, const T *src, int 
   #pragma unroll
   for (int j = 0; j < NV; j++) {
     // lanes past the last column repeat one that this lane (or lane 0) has
+    // (accumulating, they leave the walk to the others)
     const int cj = act[j] ? col0 + j * G * V : act[0] ? col0 : col0 - lane * V;
     Sj[j] = (const char *)(src + cj);
     Dj[j] = (char *)(a.dst + cj) - ldd;
@@ -194,7 +195,6 @@ __global__ void __launch_bounds__(TW_T, (ADDC || V * NV > 4 ? 3 : 4)) seg_tile_k
   const int n = min(TILE, a.nnz - ts), te = ts + n;
   const uint64_t strm = policy_stream();
   const int lane = tid & (G - 1), g = tid / G;
-  const unsigned mask = G >= 32 ? 0xffffffffu : (((1u << (G & 31)) - 1u) << (wl & ~(G - 1)));
   const int col0 = phase * COLS + lane * V;
   bool act[NV];
   #pragma unroll
@@ -265,7 +265,8 @@ __global__ void __launch_bounds__(TW_T, (ADDC || V * NV > 4 ? 3 : 4)) seg_tile_k
                                                                                    stail, lane, col0, act, strm);
   };
   // (accumulating is defined for sums only)
-  if (ADDC || a.reduce == SS_SUM) hr = a.kahan ? walk(Op<SEG_KADD>(), Op<0>()) : walk(Op<SEG_ADD>(), Op<0>());
+  if (ADDC && !act[0]) hr = 0;
+  else if (ADDC || a.reduce == SS_SUM) hr = a.kahan ? walk(Op<SEG_KADD>(), Op<0>()) : walk(Op<SEG_ADD>(), Op<0>());
   else if constexpr (!ADDC) {
     if (is_max) hr = walk(Op<SEG_MAXV>(), Op<0>());
     else hr = a.kahan ? walk(Op<SEG_KADD>(), Op<1>()) : walk(Op<SEG_ADD>(), Op<1>());

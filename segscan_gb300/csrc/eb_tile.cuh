@@ -496,6 +496,7 @@ __global__ void __launch_bounds__(TW_T, (tile_min_blocks<T, G, V, NV, ADDC>())) 
     for (int i = 0; i < 4; i++)
       if ((unsigned)c[k][i] >= (unsigned)p.K) {
         c[k][i] = -1;
+        v[k][i] = 0.f;  // (Inf and NaN times the zero row would not vanish)
         slow = true;
       }
     const int w = e + 4 * piece_of(e, p.inv_piece);

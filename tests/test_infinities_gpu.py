@@ -86,3 +86,22 @@ def test_rbsr_leaves_out_the_value_of_a_column_outside(cuda, value):
         bad[::18], bad[9::18], v[::9] = n, -1, value
         got = api.spmm(api.CsrMatrix(len(lengths), n, indptr, bad, v), B, "rbsr")
         assert torch.all((got - ref).abs() <= 1e-5 * ref.abs()), f"N={N}"
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_ebsr_leaves_out_the_value_of_a_column_outside(cuda, value):
+    """The same in the tile walk, below and above one wave of tiles."""
+    from segscan_gb300 import api
+    for lengths in ([3, 10, 70, 5, 1500], [7] * 200_000):
+        n = sum(lengths)
+        indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)).cuda()
+        cols = torch.arange(n, dtype=torch.int32, device="cuda") % 5000
+        vals = torch.ones(n, device="cuda")
+        at = torch.arange(0, n, 9, device="cuda")
+        bad, v = cols.clone(), vals.clone()
+        bad[::18], bad[9::18], v[::9] = 5000, -1, value
+        for N in (1, 4, 33, 64):
+            B = torch.rand(5000, N, device="cuda")
+            ref = api.spmm(api.CsrMatrix(len(lengths), 5000, indptr, cols, vals.index_fill(0, at, 0)), B, "ebsr")
+            got = api.spmm(api.CsrMatrix(len(lengths), 5000, indptr, bad, v), B, "ebsr")
+            assert torch.all((got - ref).abs() <= 1e-5 * ref.abs()), f"N={N} rows={len(lengths)}"

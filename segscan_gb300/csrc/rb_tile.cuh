@@ -29,12 +29,14 @@ struct RowArgs {
   void *C;
   int M, K, N, nnz;
   int rows;        // rows per group at a time
-  int block_rows;  // rows per block
+  int block_rows;  // rows per block, where the rows are about even
+  long long share;  // cost of a block above which they are not (0: not looked at)
   int kahan;
   float keep_frac;
 };
 
 constexpr int ROW_CAP = 64;  // nonzeros a group stages
+constexpr int ROW_COST = 2;  // a row's own cost (its store, the walk's bookkeeping), in nonzeros
 
 template <typename T, typename TC, int G, int V, int NV, bool ADDC>
 struct RowWalk {
@@ -102,7 +104,9 @@ struct RowWalk {
 };
 
 // A block per SM walks a contiguous range of rows, its groups side by side, so
-// that rows with near columns share the SM's L1.
+// that rows with near columns share the SM's L1.  The ranges have equal numbers
+// of rows, or, where one of those costs more than a.share, equal cost: rows
+// whose lengths follow their index would leave most SMs waiting for a few.
 template <typename T, typename TC, int G, int V, int NV, bool ADDC>
 __global__ void __launch_bounds__(ADDC ? 768 : 1024, 1) rb_tile_kernel(RowArgs a) {
   constexpr int COLS = G * V * NV, CAP = ROW_CAP, PAD = CAP + 4, IT = CAP / G;
@@ -119,19 +123,67 @@ __global__ void __launch_bounds__(ADDC ? 768 : 1024, 1) rb_tile_kernel(RowArgs a
   for (int j = 0; j < NV; j++) act[j] = col0 + j * G * V < a.N;
   RowWalk<T, TC, G, V, NV, ADDC> w(a, lane, col0, act);
   auto clamped = [&](int r) { return max(0, min(__ldg(a.indptr + r), a.nnz)); };
-  const long long b_lo = (long long)blockIdx.x * a.block_rows;
-  const long long b_hi = min(b_lo + a.block_rows, (long long)a.M);
+  // this block's rows and the rows of a unit (in shared memory: the walk needs
+  // the registers)
+  __shared__ int s_rows[3];
+  __shared__ int s_next;
+  const int blocks = gridDim.x;
+  if (tid < 2) s_rows[tid] = (int)min((long long)(blockIdx.x + tid) * a.block_rows, (long long)a.M);
+  if (tid == 0) { s_rows[2] = a.rows; s_next = NG; }
+  if (a.share) {
+    auto at_block = [&](int b) { return (int)min((long long)b * a.block_rows, (long long)a.M); };
+    bool over = false;  // every block looks at all of them, and so decides alike
+    for (int b = tid; b <= blocks; b += blockDim.x) {
+      const int r = at_block(b), p = clamped(r);
+      smem[b] = p;
+      if (b < blocks) {
+        const int r1 = at_block(b + 1);
+        over |= (long long)clamped(r1) - p + (long long)ROW_COST * (r1 - r) > a.share;
+      }
+    }
+    if (__syncthreads_or(over)) {
+      // cut where the cost of the rows before reaches the block's part of it:
+      // first among the rows looked at, then between two of them
+      const int part = blockIdx.x + (tid >> 5);
+      if (tid < 64 && part < blocks) {
+        const long long key = part * (a.nnz + (long long)ROW_COST * a.M) / blocks;
+        int lo = 0, hi = blocks;  // the first at or past it is in [lo, hi]
+        auto narrow = [&](auto cost) {
+          while (lo < hi) {
+            const int at = lo + (int)((long long)(hi - lo) * wl / 32);
+            const unsigned m = __ballot_sync(0xffffffffu, cost(at) >= key);
+            const int f = m ? __ffs(m) - 1 : 32;
+            const int below = __shfl_sync(0xffffffffu, at, max(f - 1, 0)), past = __shfl_sync(0xffffffffu, at, f & 31);
+            if (f < 32) hi = past;
+            if (f > 0) lo = below + 1;
+          }
+        };
+        narrow([&](int b) { return smem[b] + (long long)ROW_COST * at_block(b); });
+        hi = at_block(lo);
+        lo = lo > 0 ? at_block(lo - 1) : 0;
+        narrow([&](int r) { return clamped(r) + (long long)ROW_COST * r; });
+        if (wl == 0) s_rows[tid >> 5] = lo;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        // units that about fill a stage at these rows' mean length, and some
+        // for every group
+        const int rows = s_rows[1] - s_rows[0];
+        const int nnz = clamped(s_rows[1]) - clamped(s_rows[0]);
+        s_rows[2] = max(1, min(min(G, rows / NG), (int)((long long)ROW_CAP * rows / max(nnz, 1))));
+      }
+    }
+  }
   // groups take the block's rows from a counter, so a long row holds up only
   // the group that has it
-  __shared__ int s_next;
-  if (tid == 0) s_next = NG;
   __syncthreads();
   for (int unit = g;;) {
-    const long long r_at = b_lo + (long long)unit * a.rows;
+    const int b_hi = s_rows[1], rows = s_rows[2];
+    const long long r_at = s_rows[0] + (long long)unit * rows;
     if (r_at >= b_hi) break;
     if (lane == 0) unit = atomicAdd(&s_next, 1);
     unit = __shfl_sync(mask, unit, 0, G);
-    const int r0 = (int)r_at, nr = (int)min((long long)a.rows, b_hi - r_at);
+    const int r0 = (int)r_at, nr = min(rows, b_hi - r0);
     // the rows' pointers, a row per lane (at most G rows at a time)
     int rs = 0, re = 0;
     if (lane < nr) {

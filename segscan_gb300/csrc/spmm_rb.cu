@@ -414,14 +414,21 @@ ss_status launch_rbsr(const SpmmCall &c, const RbGeom &geom, cudaStream_t s) {
   const long long units = ceil_div(c.M, a.rows), blocks = std::min((long long)sm_count(), units);
   const long long per = (units + blocks - 1) / blocks;  // units per block
   a.block_rows = (int)std::min((long long)c.M, per * a.rows);
+  const long long grid = ceil_div(c.M, a.block_rows);
   const int most = addc ? 768 : 1024;
+  // Ranges of equal cost where one of equal rows costs an eighth above the mean
+  // (300 K rows of 1 to 31 in order, N = 64: 172 -> 107 us; one row in ten of
+  // 100, those first: 482 -> 131 us).  Looking costs about a microsecond (even
+  // rows 107.3 -> 108.7 us), so not where a full block has a unit per group at
+  // most (20 K rows: even 10.6 and 12.4 us, in order 14.2 and 14.5).
+  a.share = per * g.G > most ? (c.nnz + (long long)ROW_COST * c.M) / grid * 9 / 8 + 1 : 0;
   const int threads = (int)std::min((long long)most, (per * g.G + 31) / 32 * 32);
   const int NG = threads / g.G;
   const size_t group_smem = (size_t)3 * (ROW_CAP + 4) * 4;
   const ss_status st = allow_smem(fn, group_smem * (most / g.G), "rbsr shared memory");
   if (st) return st;
   void *args[] = {&a};
-  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)ceil_div(c.M, a.block_rows), (unsigned)g.phases, 1),
+  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)grid, (unsigned)g.phases, 1),
                                    dim3(threads, 1, 1), args, group_smem * NG, s);
   return e == cudaSuccess ? SS_OK : cuda_fail(e, "rbsr launch");
 }

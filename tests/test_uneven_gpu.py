@@ -58,3 +58,41 @@ def test_time_of_rows_in_order(cuda):
         plan, B, C = api.SpmmPlan(A, N, "rbsr"), torch.rand(M, N, device="cuda"), torch.empty(M, N, device="cuda")
         times.append(shortest(lambda: plan.run(B, C)))
     assert times[0] <= 1.6 * times[1], times
+
+
+def test_time_of_one_long_row(cuda):
+    """One row of 4.6 M nonzeros against a hundred of 46 K (767 and 175 us with four heads in flight)."""
+    from segscan_gb300 import api
+    K, n, N = 200_000, 4_600_000, 64
+    cols = torch.randint(0, K, (n,), device="cuda", dtype=torch.int32)
+    vals, B = torch.rand(n, device="cuda"), torch.rand(K, N, device="cuda")
+    times = []
+    for M in (1, 100):
+        A = api.CsrMatrix(M, K, torch.arange(0, n + 1, n // M, dtype=torch.int32, device="cuda"), cols, vals)
+        plan, C = api.SpmmPlan(A, N, "ebsr"), torch.empty(M, N, device="cuda")
+        times.append(shortest(lambda: plan.run(B, C)))
+    assert times[0] <= 3.6 * times[1], times
+
+
+@pytest.mark.parametrize("reduce", ["sum", "mean", "max"])
+@pytest.mark.parametrize("N", [1, 4, 33, 64])
+def test_segments_over_many_tiles(cuda, N, reduce):
+    """Last tiles one, a few, 31 to 33 and hundreds of tiles away; whole numbers, so every order of the
+    additions gives the same sum (below 2^24)."""
+    from segscan_gb300 import api
+    tile = {1: 2048, 4: 2048, 33: 1024, 64: 1024}[N]  # elements of a full tile, at most
+    lengths = [5, tile * 3 + 1, tile * 30, 2, tile * 31 + 7, tile * 32, tile * 33 - 1, 0, tile * 300, 9, tile, tile]
+    n, M = sum(lengths), len(lengths)
+    index = torch.repeat_interleave(torch.arange(M), torch.tensor(lengths)).int().cuda()
+    src = torch.randint(-8, 9, (n, N), generator=torch.Generator().manual_seed(N)).float().cuda()
+    got = api.segment(src, index, M, reduce, "sr").double()
+    want = torch.zeros(M, N, dtype=torch.float64, device="cuda")
+    if reduce == "max":
+        want = torch.stack([x.amax(0) if len(x) else want[0] for x in src.double().split(lengths)])
+    else:
+        want.index_add_(0, index.long(), src.double())
+    if reduce == "mean":
+        want /= torch.tensor(lengths, device="cuda").clamp(min=1)[:, None]
+        assert torch.all((got - want).abs() <= 2.0 ** -24 * want.abs())  # one division, rounded
+    else:
+        assert torch.equal(got, want)

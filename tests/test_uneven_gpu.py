@@ -74,6 +74,20 @@ def test_time_of_one_long_row(cuda):
     assert times[0] <= 3.6 * times[1], times
 
 
+def test_time_of_one_long_segment(cuda):
+    """One segment of 30 M elements against 300 of 100 K: what grew with the square of the tiles took
+    3287 and 358 us."""
+    from segscan_gb300 import api
+    n, N = 30_000_000, 4
+    src = torch.rand(n, N, device="cuda")
+    times = []
+    for M in (1, 300):
+        index = (torch.arange(n, device="cuda") * M // n).int()
+        out = torch.empty(M, N, device="cuda")
+        times.append(shortest(lambda: api.segment(src, index, M, "sum", "sr", out=out)))
+    assert times[0] <= 6.0 * times[1], times
+
+
 @pytest.mark.parametrize("reduce", ["sum", "mean", "max"])
 @pytest.mark.parametrize("N", [1, 4, 33, 64])
 def test_segments_over_many_tiles(cuda, N, reduce):

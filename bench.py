@@ -723,8 +723,8 @@ def run_ours(args):
                      "frac": per_gpu / peak, "peak_kind": peak_kind,
                      "traffic": traffic_from_profiles(kernel_file),
                      "gather_upper_bound_bytes": A.nnz * N * 4 + A.nnz * 8 + (A.nrow + 1) * 4 + A.nrow * N * 4,
-                     "kernel": (f"{strategy} SpMM step (walk with in-kernel carry assembly)" if strategy == "ebsr"
-                                else f"{strategy} SpMM step"),
+                     "kernel": (f"{strategy} SpMM step (rows of the tiles, tile walk, straddling rows)"
+                                if strategy == "ebsr" else f"{strategy} SpMM step"),
                      "bytes_per_launch": nbytes},
         "e2e": {"value": nbytes / t_e2e / 1e9, "unit": UNIT, "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": t_e2e * 1e3, "pinned_copy_gbs": copy_gbs},

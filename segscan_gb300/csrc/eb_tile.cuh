@@ -30,8 +30,10 @@
 // skips columns outside [0, K).
 //
 // What bounds it (power-law 1e6 x 1e6, 4.6 M nonzeros): at N = 64 FP32 the
-// gathered rows, 1.13 GB of DRAM traffic at 5.5 TB/s; with 16-bit storage
-// and at small N the issue of about 35 instructions per gathered vector.
+// gathered rows, 1.16 GB of DRAM traffic at 5.96 TB/s (195 us); with BF16
+// storage 0.59 GB at 4.2 TB/s and 65 instructions per 32 gathered vectors
+// (142 us, issue 48 % busy), at N = 4 the latency of a tile's steps (61 us,
+// issue 35 % busy, 40 % of the warp slots in use).
 #pragma once
 
 #include "eb_common.cuh"
@@ -658,8 +660,6 @@ struct TileGeom {
 // vmax: elements per vector that the alignment of B and C allows; seg: the
 // segment walk, whose rows stream instead of being gathered
 TileGeom tile_geom(int N, int nnz, int dtype, int vmax, bool seg = false);
-// Launches the walk of `a` (a.items * a.phases blocks, `smem` bytes each).
-// after_rows: right after tile_rows_kernel on the stream, which it overlaps.
 // What fix_kernel needs of one matrix (or segment reduction).
 struct TileFix {
   const int2 *span;
@@ -676,6 +676,8 @@ struct FixArgs {
 };
 // Launched right after the walk.
 ss_status run_fix(int c_dtype, FixArgs &a, int vmax, cudaStream_t s);
+// Launches the walk of `a` (a.items * a.phases blocks, `smem` bytes each).
+// after_rows: right after tile_rows_kernel on the stream, which it overlaps.
 ss_status run_tile(int val_dtype, int c_dtype, const TileGeom &g, size_t smem, TileArgs &a, bool after_rows,
                    cudaStream_t s);
 

@@ -15,8 +15,8 @@
 //
 // us, a row per team before -> staged: Poisson 200 K x 16, N = 64 94 -> 71;
 // 200 K x 1.5, N = 32 31 -> 21; banded 120 K x 20, N = 128 BF16 97 -> 69,
-// N = 64 FP32 57 -> 55.  The last is bound by L2: 614 MB of gathered rows at
-// 11 TB/s.
+// N = 64 FP32 57 -> 54.  In the last L1 serves 56 % of the sectors (614 MB of
+// gathered rows) and L2 the other 301 MB at 5.7 TB/s; issue is 50 % busy.
 #pragma once
 
 #include "eb_tile.cuh"

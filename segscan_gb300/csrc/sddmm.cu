@@ -132,10 +132,11 @@ __global__ void __launch_bounds__(256, 4) sddmm_warp_kernel(SddmmArgs a) {
     auto row_of = [&](int p) -> int {
       for (;;) {
         const int cnt = __popc(group_ballot(mask, win <= p, L));
-        if (cnt < L) return min(max(wb + cnt - 1, 0), a.M - 1);
+        // (a window that holds indptr[M] <= p: nonzeros that follow the last
+        // row, as dropped edges do)
+        if (cnt < L || wb + L - 1 >= a.M) return min(max(wb + cnt - 1, 0), a.M - 1);
         // every row start in the window is <= p: p's row is the last one or
-        // later; slide the window to it (wb + L - 1 < M here, since indptr[M]
-        // = nnz > p)
+        // later; slide the window to it
         wb += L - 1;
         win = __ldg(a.indptr + min(wb + lane, a.M));
       }

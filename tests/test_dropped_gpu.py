@@ -64,3 +64,20 @@ def test_gradient_of_B(cuda, scratch, N):
     autograd.spmm(A, A.values, B).backward(torch.from_numpy(dC).cuda())
     want, terms = expect(cols, rows, vals, n, dC)
     assert np.all(np.abs(B.grad.double().cpu().numpy() - want) <= 1e-5 * terms + 1e-30)
+
+
+@pytest.mark.parametrize("N", [4, 64, 100, 128, 256])
+@pytest.mark.parametrize("nrow,nnz,dropped", [(5000, 9000, 700), (41, 300, 299), (50, 50, 50), (5000, 300_000, 6000)])
+def test_gradient_of_the_values(cuda, N, nrow, nnz, dropped):
+    """SDDMM: 0 for entries that follow the last row, whose columns are -1."""
+    from segscan_gb300 import api
+    rows, cols = dropping(nnz, nrow, dropped)
+    A, perm = api.coo_to_csr(nrow, torch.from_numpy(rows).cuda(), torch.from_numpy(cols).cuda(), ncol=nrow)
+    rng = np.random.default_rng(3)
+    dC, B = (rng.uniform(-1, 1, (nrow, N)).astype(np.float32) for _ in "ab")
+    got = api.sddmm(A, torch.from_numpy(dC).cuda(), torch.from_numpy(B).cuda()).double().cpu().numpy()
+    kept = perm.cpu().numpy()[:nnz - dropped]
+    want = np.einsum("ij,ij->i", dC[rows[kept]].astype(np.float64), B[cols[kept]])
+    terms = np.einsum("ij,ij->i", np.abs(dC[rows[kept]]).astype(np.float64), np.abs(B[cols[kept]]))
+    assert np.all(np.abs(got[:nnz - dropped] - want) <= 1e-5 * terms + 1e-30)
+    assert np.all(got[nnz - dropped:] == 0)

@@ -90,7 +90,8 @@ __device__ __forceinline__ bool row_ends_in_chunk(const EbArgs &a, const ChunkIn
   if (ci.ce >= a.nnz) return true;
   if (SEG) return __ldg(a.index + ci.ce) != row;
   if ((unsigned)row >= (unsigned)a.M) return true;
-  return __ldg(a.indptr + row + 1) <= ci.ce;
+  // (nonzeros past indptr[M], as dropped edges are, count as the last row's)
+  return row < a.M - 1 && __ldg(a.indptr + row + 1) <= ci.ce;
 }
 
 // Writes zeros to rows [lo, hi] (clamped to the output) for this lane's

@@ -81,3 +81,20 @@ def test_gradient_of_the_values(cuda, N, nrow, nnz, dropped):
     terms = np.einsum("ij,ij->i", np.abs(dC[rows[kept]]).astype(np.float64), np.abs(B[cols[kept]]))
     assert np.all(np.abs(got[:nnz - dropped] - want) <= 1e-5 * terms + 1e-30)
     assert np.all(got[nnz - dropped:] == 0)
+
+
+@pytest.mark.parametrize("strategy", ["ebpr", "rbpr", "rbsr"])
+@pytest.mark.parametrize("N,nnz,dropped", [(4, 9000, 700), (33, 9000, 6000), (64, 300_000, 1), (64, 300_000, 9000)])
+def test_other_strategies(cuda, scratch, strategy, N, nnz, dropped):
+    """(the last row has nonzeros here, and chunks of dropped entries follow its own)"""
+    from segscan_gb300 import api
+    nrow = 5000
+    rows, cols = dropping(nnz, nrow, dropped)
+    rows[np.flatnonzero(rows < nrow)[:7]] = nrow - 1
+    vals = np.random.default_rng(1).uniform(-1, 1, nnz).astype(np.float32)
+    A, _ = api.coo_to_csr(nrow, torch.from_numpy(rows).cuda(), torch.from_numpy(cols).cuda(), ncol=nrow,
+                          values=torch.from_numpy(vals).cuda())
+    B = np.random.default_rng(7).uniform(-1, 1, (nrow, N)).astype(np.float32)
+    got = api.spmm(A, torch.from_numpy(B).cuda(), strategy).double().cpu().numpy()
+    want, terms = expect(rows, cols, vals, nrow, B)
+    assert np.all(np.abs(got - want) <= 1e-5 * terms + 1e-30)

@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(512, SS_SR_MIN_BLOCKS) batched_kernel(const ch
     const int chunk = item - mt.item_begin;
     a.M = mt.M;
     a.K = mt.K;
-    a.nnz = mt.nnz;
+    // row-balanced items end with the last row (dropped edges follow it)
+    a.nnz = mt.rows_per_item > 0 ? __ldg(mt.indptr + mt.M) : mt.nnz;
     a.indptr = mt.indptr;
     a.cols = mt.indices;
     a.vals = mt.vals;
@@ -129,7 +130,10 @@ __global__ void __launch_bounds__(512, SS_SR_MIN_BLOCKS) batched_kernel(const ch
       const int r0 = chunk * mt.rows_per_item;
       cs = __ldg(mt.indptr + r0);
       ce = __ldg(mt.indptr + min(mt.M, r0 + mt.rows_per_item));
-      if (cs == ce) continue;  // empty rows only: the item holding the next nonzero zeroes them
+      if (cs == ce) {  // empty rows only: the item holding the next nonzero zeroes them
+        if (a.nnz == 0 && chunk == 0) zero_rows<TC, V, NV>(a, 0, a.M - 1, col0, act, strm);
+        continue;
+      }
     } else {
       cs = chunk * mt.chunk;
       ce = min(cs + mt.chunk, mt.nnz);

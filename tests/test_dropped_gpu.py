@@ -98,3 +98,23 @@ def test_other_strategies(cuda, scratch, strategy, N, nnz, dropped):
     got = api.spmm(A, torch.from_numpy(B).cuda(), strategy).double().cpu().numpy()
     want, terms = expect(rows, cols, vals, nrow, B)
     assert np.all(np.abs(got - want) <= 1e-5 * terms + 1e-30)
+
+
+@pytest.mark.parametrize("N", [4, 33, 64])
+@pytest.mark.parametrize("strategy", ["rbsr", "ebsr"])
+def test_batched(cuda, strategy, N):
+    """Trailing empty rows are written too; the last matrix has dropped edges only."""
+    from segscan_gb300 import api, autotune
+    from segscan_gb300.batched import BatchedSpMM
+    mats, Bs, wants = [], [], []
+    for i, (nrow, nnz, dropped) in enumerate([(5000, 9000, 700), (60, 300, 1), (900, 40_000, 9000), (50, 70, 70)]):
+        rows, cols = dropping(nnz, nrow, dropped, seed=i)
+        vals = np.random.default_rng(1).uniform(-1, 1, nnz).astype(np.float32)
+        B = np.random.default_rng(7).uniform(-1, 1, (nrow, N)).astype(np.float32)
+        mats.append(api.coo_to_csr(nrow, torch.from_numpy(rows).cuda(), torch.from_numpy(cols).cuda(), ncol=nrow,
+                                   values=torch.from_numpy(vals).cuda())[0])
+        Bs.append(torch.from_numpy(B).cuda())
+        wants.append(expect(rows, cols, vals, nrow, B))
+    outs = BatchedSpMM(mats, Bs, knobs=autotune.batch_knobs(mats, N), strategies=[strategy] * len(mats)).run()
+    for got, (want, terms) in zip(outs, wants):
+        assert np.all(np.abs(got.double().cpu().numpy() - want) <= 1e-5 * terms + 1e-30)

@@ -153,6 +153,10 @@ __device__ __forceinline__ void flush_row(const EbArgs &a, const ChunkInfo &ci, 
   }
 }
 
+// indptr[r], and nnz from the last row's end on: nonzeros past indptr[M] (as
+// dropped edges are, their columns outside the matrix) count as the last row's.
+__device__ __forceinline__ int row_ptr(const EbArgs &a, int r) { return r < a.M ? __ldg(a.indptr + r) : a.nnz; }
+
 // V floats from a carry slot written by other blocks in this launch: read
 // at L2 (ld.global.cg), never from a possibly stale L1 line.
 template <int V>
@@ -184,7 +188,7 @@ template <typename TC, int V, int NV>
 __device__ __forceinline__ void carry_arrive(const EbArgs &a, int r, int lane, int G, unsigned mask, int col0,
                                           const bool (&act)[NV], uint64_t pol) {
   const int o = __ldg(a.indptr + r) / a.chunk;
-  const int l = (__ldg(a.indptr + r + 1) - 1) / a.chunk;
+  const int l = (row_ptr(a, r + 1) - 1) / a.chunk;
   int *cnt = a.carry_cnt + (size_t)o * gridDim.y + blockIdx.y;
   __threadfence();  // this lane's slot stores are visible before the count moves
   __syncwarp(mask);

@@ -219,7 +219,7 @@ __device__ __forceinline__ bool sr_spmm_walk(const EbArgs &a, int chunk, int cs,
   auto win_fill = [&](int base) {
     __syncwarp(mask);
     win_base = base;
-    for (int i = lane; i < L.W; i += G) st.win[i] = __ldg(a.indptr + min(base + i, a.M));
+    for (int i = lane; i < L.W; i += G) st.win[i] = row_ptr(a, base + i);
     __syncwarp(mask);
   };
   auto wget = [&](int r) -> int {
@@ -501,7 +501,7 @@ __device__ __forceinline__ bool sr_spmm_chunk(const EbArgs &a, int chunk, int cs
   const int lb = group_lower_bound(a.indptr, a.M, cs, lane, G, mask);
   const int base = lb > 0 ? lb - 1 : 0;
   __syncwarp(mask);
-  for (int i = lane; i < L.W; i += G) st.win[i] = __ldg(a.indptr + min(base + i, a.M));
+  for (int i = lane; i < L.W; i += G) st.win[i] = row_ptr(a, base + i);
   __syncwarp(mask);
   return sr_spmm_walk<T, TC, V, NV>(a, chunk, cs, ce, nst, lb, base, lane, mask, st, L, col0, act, keep, strm);
 }

@@ -118,3 +118,21 @@ def test_batched(cuda, strategy, N):
     outs = BatchedSpMM(mats, Bs, knobs=autotune.batch_knobs(mats, N), strategies=[strategy] * len(mats)).run()
     for got, (want, terms) in zip(outs, wants):
         assert np.all(np.abs(got.double().cpu().numpy() - want) <= 1e-5 * terms + 1e-30)
+
+
+@pytest.mark.parametrize("N,nnz,dropped", [(4, 9000, 700), (33, 9000, 6000), (64, 300_000, 1), (64, 300_000, 20_000)])
+def test_group_walk(cuda, scratch, N, nnz, dropped):
+    """ebsr with runs above 2048 nonzeros: chunks that hold the last row and dropped entries, or these alone."""
+    from segscan_gb300 import api
+    nrow = 5000
+    knobs = api.make_knobs("ebsr", N, thread_nz=4096)
+    for last in (0, 7):
+        rows, cols = dropping(nnz, nrow, dropped)
+        rows[np.flatnonzero(rows < nrow)[:last]] = nrow - 1
+        vals = np.random.default_rng(1).uniform(-1, 1, nnz).astype(np.float32)
+        A, _ = api.coo_to_csr(nrow, torch.from_numpy(rows).cuda(), torch.from_numpy(cols).cuda(), ncol=nrow,
+                              values=torch.from_numpy(vals).cuda())
+        B = np.random.default_rng(7).uniform(-1, 1, (nrow, N)).astype(np.float32)
+        got = api.spmm(A, torch.from_numpy(B).cuda(), "ebsr", knobs=knobs).double().cpu().numpy()
+        want, terms = expect(rows, cols, vals, nrow, B)
+        assert np.all(np.abs(got - want) <= 1e-5 * terms + 1e-30)

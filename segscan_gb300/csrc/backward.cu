@@ -211,6 +211,13 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 1) fused_bwd_kernel(BwdArgs
   while (k < r_hi) next_row();
 }
 
+// The walk writes dvals at the nonzeros that A^T holds.  Where A has others
+// (columns outside the matrix, edges past the last row), dvals starts as 0.
+__global__ void __launch_bounds__(256) zero_dropped_kernel(const int32_t *__restrict__ t_end, int nnz, float *dvals) {
+  if (__ldg(t_end) >= nnz) return;
+  for (long long q = blockIdx.x * 256ll + threadIdx.x; q < nnz; q += gridDim.x * 256ll) dvals[q] = 0.f;
+}
+
 template <typename T, typename TC, bool WARP>
 static void *bwd_ptr_w(int V, int NV) {
   if (NV == 1) {
@@ -293,6 +300,12 @@ extern "C" ss_status ss_spmm_backward(const ss_csr *AT, const int32_t *perm, con
   a.chunk = (int)chunk;
   a.groups = (int)groups;
   const long long blocks = (groups + groups_per_block - 1) / groups_per_block;
+  if (nnz > 0) {
+    const ss_status st = launch("fused backward dropped nonzeros", zero_dropped_kernel,
+                                std::min((nnz - 1) / 256 + 1, sm_count() * 8), 256, 0, (cudaStream_t)stream,
+                                AT->indptr + K, nnz, dvals);
+    if (st != SS_OK) return st;
+  }
   void *args[] = {&a};
   e = cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(threads), args, 0, (cudaStream_t)stream);
   return e == cudaSuccess ? SS_OK : cuda_fail(e, "fused backward launch");

@@ -136,3 +136,26 @@ def test_group_walk(cuda, scratch, N, nnz, dropped):
         got = api.spmm(A, torch.from_numpy(B).cuda(), "ebsr", knobs=knobs).double().cpu().numpy()
         want, terms = expect(rows, cols, vals, nrow, B)
         assert np.all(np.abs(got - want) <= 1e-5 * terms + 1e-30)
+
+
+@pytest.mark.parametrize("N", [4, 64, 128])
+def test_both_gradients(cuda, N):
+    """One walk over A^T gives both; nonzeros that A^T does not hold get 0."""
+    from segscan_gb300 import api, autograd
+    nnz, n, dropped = 60_000, 5000, 6000
+    cols, rows = dropping(nnz, n, dropped)
+    rows = np.sort(rows)
+    indptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int32)
+    vals = np.random.default_rng(1).uniform(-1, 1, nnz).astype(np.float32)
+    rng = np.random.default_rng(3)
+    dC, Bh = (rng.uniform(-1, 1, (n, N)).astype(np.float32) for _ in "ab")
+    A = api.CsrMatrix(n, n, torch.from_numpy(indptr).cuda(), torch.from_numpy(cols).cuda(), None)
+    v = torch.from_numpy(vals).cuda().requires_grad_(True)
+    B = torch.from_numpy(Bh).cuda().requires_grad_(True)
+    autograd.spmm(A, v, B).backward(torch.from_numpy(dC).cuda())
+    kept = cols < n
+    want = np.where(kept, np.einsum("ij,ij->i", dC[rows].astype(np.float64), Bh[np.where(kept, cols, 0)]), 0)
+    terms = np.einsum("ij,ij->i", np.abs(dC[rows]).astype(np.float64), np.abs(Bh[np.where(kept, cols, 0)]))
+    assert np.all(np.abs(v.grad.double().cpu().numpy() - want) <= 1e-5 * terms)
+    want, terms = expect(cols, rows, vals, n, dC)
+    assert np.all(np.abs(B.grad.double().cpu().numpy() - want) <= 1e-5 * terms + 1e-30)

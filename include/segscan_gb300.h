@@ -77,7 +77,9 @@ typedef enum {
  * (__guard_load_default_one, test-cg/include/util/check.cuh:104-111). */
 typedef struct {
   int32_t nrow, ncol, nnz;
-  const int32_t *indptr;  /* [nrow + 1], indptr[0] = 0, indptr[nrow] = nnz */
+  const int32_t *indptr;  /* [nrow + 1], indptr[0] = 0, indptr[nrow] = nnz (less
+                             where dropped edges, with column -1, follow the
+                             last row, as ss_coo_to_csr leaves them) */
   const int32_t *indices; /* [nnz], column of each nonzero, in [0, ncol)   */
   const void *values;     /* [nnz] of value_dtype, or NULL                 */
   int32_t value_dtype;    /* ss_dtype                                       */

@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(1024) eb_pr_kernel(EbArgs a) {
   const int col0 = blockIdx.y * a.col_tile + cg * V;
   bool act[1] = {col0 < a.N};
   const uint64_t keep = policy_keep(a.keep_frac), strm = policy_stream();
+  const bool gathers = act[0] && a.K > 0;
   const bool is_max = SEG && a.reduce == SS_MAX;
   const float ident = is_max ? -INFINITY : 0.f;
   const int stride = gridDim.x * a.workers_per_block;
@@ -88,14 +89,14 @@ __global__ void __launch_bounds__(1024) eb_pr_kernel(EbArgs a) {
       int c = 0;
       float v = 0.f;
       float b[V];
+      bool in = true;  // a column outside the matrix adds nothing, whatever its value
       if (SEG) {
         c = p;
-        v = 1.f;
       } else {
         c = c_next;
         v = v_next;
-        if ((unsigned)c >= (unsigned)a.K) { c = 0; v = 0.f; }
-        if (live && act[0]) load_vec<T, V>(B + (int64_t)c * a.N + col0, b, keep);
+        in = (unsigned)c < (unsigned)a.K;
+        if (live && gathers) load_vec<T, V>(B + (int64_t)(in ? c : 0) * a.N + col0, b, keep);
         const int pn = p + tile;
         if (pn < ci.ce) {
           c_next = ld_idx(a.cols + pn, strm);
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(1024) eb_pr_kernel(EbArgs a) {
         }
         if (act[0]) {
           #pragma unroll
-          for (int i = 0; i < V; i++) x[0][i] = is_max ? b[i] : v * b[i];
+          for (int i = 0; i < V; i++) x[0][i] = SEG ? b[i] : in ? v * b[i] : 0.f;
         }
         cnt = 1;
       }

@@ -275,7 +275,7 @@ __device__ __forceinline__ bool sr_spmm_walk(const EbArgs &a, int chunk, int cs,
       return false;
     }
     const int32_t *scol = st.col + b * L.S;
-    const T *sval = reinterpret_cast<const T *>(st.val + b * L.S * L.vs);
+    T *sval = reinterpret_cast<T *>(st.val + b * L.S * L.vs);
     int32_t *sinfo = st.info + b * L.S;
 
     // the window must hold the starts of every row this tile touches and of
@@ -297,7 +297,13 @@ __device__ __forceinline__ bool sr_spmm_walk(const EbArgs &a, int chunk, int cs,
         int zlo = 0, zhi = -1;
         bool kah = false;
         if (e < n) {
-          bad |= (unsigned)scol[e] >= (unsigned)a.K;
+          if ((unsigned)scol[e] >= (unsigned)a.K) {
+            bad = true;
+            if (!ones) {
+              sval[e] = Elem<T>::from_f(0.f);  // Inf times the zero row would not vanish
+              fence_async_smem();              // before a bulk copy refills the buffer
+            }
+          }
           const int p = sb + e;
           int lo = c0 + 1, hi = L.W - 1;
           while (lo < hi) {
@@ -453,7 +459,7 @@ __device__ __forceinline__ bool sr_spmm_walk(const EbArgs &a, int chunk, int cs,
           next_start = ns;
           kah = next_start - wget(cur) > a.kahan;
         }
-        const float v = ones ? 1.f : Elem<T>::to_f(sval[q]);
+        const float v = (unsigned)c >= (unsigned)a.K ? 0.f : ones ? 1.f : Elem<T>::to_f(sval[q]);
         add_row<V, NV>(acc, comp, v, bq, kah);
         open = true;
       }

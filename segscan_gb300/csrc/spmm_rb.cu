@@ -106,7 +106,7 @@ __device__ __forceinline__ void rbsr_row(const RbArgs &a, int s, int e, int lane
     if (p < e) {
       mc = ld_idx(a.indices + p, strm);
       mv = load_val<T>(vals, p, strm);
-      if ((unsigned)mc >= (unsigned)a.K) { mc = 0; mv = 0.f; }
+      if ((unsigned)mc >= (unsigned)a.K) mc = -1;  // adds nothing
     }
     const int cnt = min(L, e - base);
     for (int q = 0; q < cnt; q += 4) {
@@ -120,7 +120,7 @@ __device__ __forceinline__ void rbsr_row(const RbArgs &a, int s, int e, int lane
       }
       #pragma unroll
       for (int u = 0; u < 4; u++) {
-        const bool live = q + u < cnt;
+        const bool live = q + u < cnt && c[u] >= 0;
         #pragma unroll
         for (int j = 0; j < NV; j++) {
           if (live && act[j]) {

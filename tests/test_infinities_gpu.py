@@ -105,3 +105,24 @@ def test_ebsr_leaves_out_the_value_of_a_column_outside(cuda, value):
             ref = api.spmm(api.CsrMatrix(len(lengths), 5000, indptr, cols, vals.index_fill(0, at, 0)), B, "ebsr")
             got = api.spmm(api.CsrMatrix(len(lengths), 5000, indptr, bad, v), B, "ebsr")
             assert torch.all((got - ref).abs() <= 1e-5 * ref.abs()), f"N={N} rows={len(lengths)}"
+
+
+@pytest.mark.parametrize("value", [1.0, np.inf, np.nan])
+@pytest.mark.parametrize("strategy,kw", SPMM + [("ebsr", dict(thread_nz=4096))])
+def test_columns_outside_add_nothing(cuda, strategy, kw, value):
+    """Whatever the value there and in any row of B that no other nonzero names (rows 0 and K - 1)."""
+    from segscan_gb300 import api
+    n = sum(LENGTHS)
+    indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(LENGTHS)]).astype(np.int32)).cuda()
+    cols = 1 + torch.arange(n, dtype=torch.int32, device="cuda")
+    vals = torch.ones(n, device="cuda")
+    bad, v = cols.clone(), vals.clone()
+    bad[::18], bad[9::18], v[::9] = n + 2, -1, value
+    at = torch.arange(0, n, 9, device="cuda")
+    for N in (4, 33, 64):
+        knobs = api.make_knobs(strategy, N, **kw) if kw else None
+        B = torch.rand(n + 2, N, device="cuda")
+        ref = api.spmm(api.CsrMatrix(len(LENGTHS), n + 2, indptr, cols, vals.index_fill(0, at, 0)), B, strategy, knobs=knobs)
+        B[0], B[n + 1] = np.inf, np.nan
+        got = api.spmm(api.CsrMatrix(len(LENGTHS), n + 2, indptr, bad, v), B, strategy, knobs=knobs)
+        assert torch.all((got - ref).abs() <= 1e-5 * ref.abs()), f"N={N}"
